@@ -65,9 +65,11 @@ int dlti_get_tmap_mn3d(CUtensorMap* out, const void* base, uint64_t N, uint64_t 
 
 #ifdef __CUDACC__
 // Launch `kernel` on `stream`, as a programmatic dependent of the previous kernel in the stream when PDL is on.
-// `rows` = token rows of the step: PDL pays off while a step is latency-bound (measured on B200, Llama-2-7B decode:
-// -7 % at 1 row, -6 % at 16, +2 % at 64), so larger steps fall back to plain stream ordering.
-constexpr long long DLTI_PDL_MAX_ROWS = 32;
+// `rows` = token rows of the step. A decode step is a chain of kernels of a few microseconds up to the largest batch that the decode
+// GEMM takes, so all of these overlap their launches: a step of 64 rows takes 860 instead of 965 us on 12 Llama layers of width 2048
+// and 655 instead of 727 us on 6 Logozen layers; at 64 rows of 4 Llama-2-7B layers, where the weights take most of it, 678 and
+// 680 us. Larger steps fall back to plain stream ordering: their kernels fill the GPU.
+constexpr long long DLTI_PDL_MAX_ROWS = 256;
 template <typename... KArgs, typename... Args>
 inline cudaError_t dlti_launch_pdl(long long rows, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                    cudaStream_t stream, Args... args) {
