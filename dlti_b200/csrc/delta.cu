@@ -35,14 +35,123 @@ __device__ __forceinline__ float step_share(const DeltaParams& p, long long row,
   return 1.f / (1.f + expf(-p.gates[row * p.g_ld + p.heads + h]));
 }
 
+// One token per sequence (decode rows), bound by the state, read and written once: a lane owns V consecutive columns, so a CTA has
+// V times the bytes in flight for the same barriers and the same loads of q and k. The order of all sums is that of the
+// token-by-token form below.
+template <typename T, int NR, int V>
+__global__ void __launch_bounds__(256, NR * V <= 32 ? 4 : 2) delta_step_kernel(const DeltaParams p, int blocks, int conv_parts) {
+  griddep_wait();
+  griddep_launch();
+  const int s = p.seq0 + blockIdx.z;
+  if ((int)blockIdx.x >= blocks) {
+    if (blockIdx.y == 0) conv_tail<T>(p, s, blockIdx.x - blocks, conv_parts);
+    return;
+  }
+  __shared__ float sk[8 * NR], sq[8 * NR], sc[3];          // sc: k . q, share, decay
+  __shared__ __align__(16) float2 part[8][32 * V];
+  const int h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = h / p.rep;
+  const int col = (blockIdx.x * 32 + lane) * V;
+  const int slot = p.sslot[s];
+  const bool live = slot >= 0 && p.ctx[s] > 1, colok = col < p.P;                  // P is a multiple of V
+  const long long row = s;
+  float* st = p.state + (((long long)(slot < 0 ? 0 : slot) * p.heads + h) * p.N + warp * NR) * p.P + col;
+  float S[NR][V];
+#pragma unroll
+  for (int i = 0; i < NR; ++i) {
+    const bool ok = live && colok && warp * NR + i < p.N;
+    if constexpr (V == 4) {
+      const float4 x = ok ? *reinterpret_cast<const float4*>(st + (long long)i * p.P) : make_float4(0.f, 0.f, 0.f, 0.f);
+      S[i][0] = x.x; S[i][1] = x.y; S[i][2] = x.z; S[i][3] = x.w;
+    } else if constexpr (V == 2) {
+      const float2 x = ok ? *reinterpret_cast<const float2*>(st + (long long)i * p.P) : make_float2(0.f, 0.f);
+      S[i][0] = x.x; S[i][1] = x.y;
+    } else {
+      S[i][0] = ok ? st[(long long)i * p.P] : 0.f;
+    }
+  }
+  const T* v = reinterpret_cast<const T*>(p.v) + row * p.v_ld + (long long)h * p.P;
+  if (warp == 0) {
+    const T* q = reinterpret_cast<const T*>(p.q) + row * p.q_ld + (long long)grp * p.N;
+    const T* k = reinterpret_cast<const T*>(p.k) + row * p.k_ld + (long long)grp * p.N;
+    constexpr int PER = (8 * NR + 31) / 32;
+    float a[PER], b[PER], kk = 0.f, qq = 0.f, kq = 0.f;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int i = lane + 32 * j;
+      a[j] = i < p.N ? Cvt<T>::to_f(k[i]) : 0.f;
+      b[j] = i < p.N ? Cvt<T>::to_f(q[i]) : 0.f;
+      kk = fmaf(a[j], a[j], kk);
+      qq = fmaf(b[j], b[j], qq);
+      kq = fmaf(a[j], b[j], kq);
+    }
+    const float rk = 1.f / sqrtf(warp_sum(kk) + UNIT_EPS), rq = 1.f / sqrtf((float)p.N) / sqrtf(warp_sum(qq) + UNIT_EPS);
+    kq = warp_sum(kq);
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if (lane + 32 * j < 8 * NR) {
+        sk[lane + 32 * j] = a[j] * rk;
+        sq[lane + 32 * j] = b[j] * rq;
+      }
+    if (lane == 0) sc[0] = kq * rk * rq;
+  } else if (threadIdx.x == 32) {
+    sc[1] = step_share(p, row, h);
+    sc[2] = decay_of(log_decay(p, row, h));
+  }
+  float vv[V], a[V], b[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) {
+    vv[j] = colok ? Cvt<T>::to_f(v[col + j]) : 0.f;
+    a[j] = b[j] = 0.f;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NR; ++i)
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      a[j] = fmaf(sk[warp * NR + i], S[i][j], a[j]);
+      b[j] = fmaf(sq[warp * NR + i], S[i][j], b[j]);
+    }
+#pragma unroll
+  for (int j = 0; j < V; ++j) part[warp][lane * V + j] = make_float2(a[j], b[j]);
+  __syncthreads();
+  const float g = sc[2];
+  float u[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) {
+    a[j] = b[j] = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const float2 x = part[w][lane * V + j];
+      a[j] += x.x;
+      b[j] += x.y;
+    }
+    u[j] = sc[1] * (vv[j] - g * a[j]);
+  }
+  if (slot >= 0 && colok) {
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      if (warp * NR + i >= p.N) break;
+      const float kr = sk[warp * NR + i];
+#pragma unroll
+      for (int j = 0; j < V; ++j) S[i][j] = fmaf(g, S[i][j], kr * u[j]);
+      if constexpr (V == 4) *reinterpret_cast<float4*>(st + (long long)i * p.P) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+      else if constexpr (V == 2) *reinterpret_cast<float2*>(st + (long long)i * p.P) = make_float2(S[i][0], S[i][1]);
+      else st[(long long)i * p.P] = S[i][0];
+    }
+  }
+  if (warp == 7 && colok) {
+    T* o = reinterpret_cast<T*>(p.out) + row * p.o_ld + (long long)h * p.P + col;
+#pragma unroll
+    for (int j = 0; j < V; ++j) o[j] = Cvt<T>::from_f(fmaf(sc[0], u[j], g * b[j]));
+  }
+}
+
 // CTA = (32 columns of P, head, sequence), 8 warps: lane = column, a warp owns the NR consecutive rows [warp * NR, ...). With the
 // old state's products k^T S and q^T S known, u and o = g q^T S + (k . q) u follow without a second pass, so a token costs one
 // exchange between the warps. TT tokens are staged at a time.
 constexpr int TT = 8;
 template <typename T, int NR>
 __global__ void __launch_bounds__(256) delta_kernel(const DeltaParams p, int slices, int conv_parts) {
-  griddep_wait();
-  griddep_launch();
   const int s = p.seq0 + blockIdx.z;
   if ((int)blockIdx.x >= slices) {
     if (blockIdx.y == 0) conv_tail<T>(p, s, blockIdx.x - slices, conv_parts);
@@ -625,17 +734,33 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) delta_chunk_kernel(con
   }
 }
 
+template <typename T, int NR, int V>
+int launch_step(const DeltaParams& p, int nseq, cudaStream_t st) {
+  const int blocks = (p.P + 32 * V - 1) / (32 * V), conv_parts = p.conv_state ? (p.conv_C + 2047) / 2048 : 0;
+  DLTI_CUDA_CHECK(dlti_launch_pdl(p.nd, delta_step_kernel<T, NR, V>, dim3(blocks + conv_parts, p.heads, nseq), dim3(256), 0, st, p, blocks, conv_parts));
+  dlti_count_launch();
+  return 0;
+}
+template <typename T, int NR>
+int dispatch_step(const DeltaParams& p, int nseq, cudaStream_t st) {
+  constexpr int MOST = NR <= 16 ? 4 : (NR == 32 ? 2 : 1);
+  const int V = step_columns(p.P, MOST, (long long)p.heads * nseq, p.state);
+  if constexpr (MOST >= 4) if (V == 4) return launch_step<T, NR, 4>(p, nseq, st);
+  if constexpr (MOST >= 2) if (V == 2) return launch_step<T, NR, 2>(p, nseq, st);
+  return launch_step<T, NR, 1>(p, nseq, st);
+}
+
 template <typename T>
 int launch_tokens(const DeltaParams& p, int nseq, cudaStream_t st) {
   const int slices = (p.P + 31) / 32;
   const int conv_parts = p.conv_state ? (p.conv_C + 2047) / 2048 : 0;
   const dim3 grid(slices + conv_parts, p.heads, nseq);
-  const long long rows = p.nd > 0 && p.seq0 + nseq <= p.nd ? p.nd : 1 << 20;     // a programmatic dependent launch only pays in decode-sized steps
 #define DELTA_CASE(NR)                                                                                           \
   if (p.N <= 8 * NR) {                                                                                           \
-    DLTI_CUDA_CHECK(dlti_launch_pdl(rows, delta_kernel<T, NR>, grid, dim3(256), 0, st, p, slices, conv_parts));   \
+    if (p.seq0 + nseq <= p.nd) return dispatch_step<T, NR>(p, nseq, st);                                         \
+    delta_kernel<T, NR><<<grid, 256, 0, st>>>(p, slices, conv_parts);                                            \
     dlti_count_launch();                                                                                         \
-    return 0;                                                                                                    \
+    return (int)cudaGetLastError();                                                                              \
   }
   DELTA_CASE(4) DELTA_CASE(8) DELTA_CASE(16) DELTA_CASE(32) DELTA_CASE(64)
 #undef DELTA_CASE

@@ -41,3 +41,11 @@ __device__ __forceinline__ void conv_tail(const Params& p, int s, int part, int 
       st[(long long)j * p.conv_C + c] = v;
     }
 }
+
+// Columns per lane: as many as the states' alignment allows, as long as no lane stays idle and the SMs have a CTA each.
+inline int step_columns(int P, int most, long long heads, const void* state) {
+  for (int V = most; V > 1; V /= 2)
+    if (P % V == 0 && P > 16 * V && ((P + 32 * V - 1) / (32 * V)) * heads >= dlti_num_sms() && (reinterpret_cast<uintptr_t>(state) & (4 * V - 1)) == 0)
+      return V;
+  return 1;
+}

@@ -1,0 +1,57 @@
+"""Kernels of decode rows whose work is cut by the sizes of a step: recurrent states moved several columns a lane, each against the
+op's restatement in plain PyTorch."""
+import pytest
+import torch
+
+from dlti_b200.ops import delta as D
+from dlti_b200.ops import stack as K
+
+pytestmark = pytest.mark.gpu
+BF16, F32 = torch.bfloat16, torch.float32
+
+
+def _rows(n, device):
+    """n decode rows; every fifth sequence is new (nothing carried), every seventh has no state slot (padding)."""
+    i = torch.arange(n, dtype=torch.int32)
+    ctx = torch.where(i % 5 == 0, torch.ones_like(i), i + 2)
+    state = torch.where(i % 7 == 3, torch.full_like(i, -1), n - 1 - i)
+    t = lambda x: x.to(device)
+    return K.Rows(t(ctx - 1), t(i), t(i.long()), t(ctx), None, torch.zeros(n, 1, dtype=torch.int32, device=device), t(state), n, 0, 64)
+
+
+def _act(x, device, dtype):
+    out = K.act(x.shape[0], x.shape[1], dtype, device)
+    return out.copy_(x)
+
+
+# four, two and one column per lane; last blocks and last rows partly filled; every row count of a warp
+SIZES = [(4, 128, 128, 40), (4, 128, 256, 40), (8, 30, 132, 40), (4, 72, 64, 40), (4, 20, 44, 80), (4, 128, 70, 40), (8, 256, 96, 40), (3, 64, 33, 60),
+         (2, 300, 40, 80), (2, 128, 128, 3)]
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("heads,N,P,n", SIZES)
+@pytest.mark.parametrize("kind", ["mamba2", "lightning", "mlstm", "delta"])
+def test_recurrences_of_decode_rows(kind, heads, N, P, n, dtype):
+    g = torch.Generator().manual_seed(N + P)
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    q, k, v, z = (rnd(n, w).to(BF16).float() for w in (heads * N, heads * N, heads * P, 2 * heads))
+    state, vec = rnd(n, heads, N, P), rnd(n, heads, 1, N + 1).repeat(1, 1, -(-P // 32), 1).flatten(2)
+    bias, A_log, skip, fall = rnd(heads), rnd(heads) * 0.5, rnd(heads), torch.rand(heads, generator=g)
+    got = {}
+    for device in ("cpu", "cuda"):
+        t = lambda x: x.to(device)
+        rows, st, vc, dt = _rows(n, device), state.to(device, copy=True), vec.to(device, copy=True), F32 if device == "cpu" else dtype
+        a = [_act(x, device, dt) for x in (q, k, v)]
+        if kind == "delta":
+            out = D.delta_scan(*a, _act(z, device, F32), t(A_log), t(bias), st, rows, heads, heads, N, P)
+        elif kind == "mlstm":
+            out = K.mlstm_scan(*a, _act(z, device, F32), t(torch.cat([bias, bias])), 15.0, st, vc, rows, heads, N, P)
+        else:
+            dec = K.Decay(const=t(fall)) if kind == "lightning" else K.Decay(dt=_act(z[:, :heads], device, dt), dt_bias=t(bias), A_log=t(A_log), D=t(skip))
+            out = K.linear_scan(*a, dec, st, rows, heads, heads, N, P, silu=kind == "lightning" and dtype == F32)
+        got[device] = out.float().cpu(), st.cpu(), vc.cpu()
+    live = (_rows(n, "cpu").state >= 0)
+    for x, y, tol in zip(got["cuda"], got["cpu"], (1e-5 if dtype == F32 else 4e-3, 1e-5, 1e-5)):     # fp32 sums; outputs rounded to 8 bits
+        x, y = (x[live], y[live]) if x.shape[0] == n and x.dim() == 2 else (x, y)                     # rows without a slot: no result
+        assert (x.double() - y.double()).norm() <= tol * y.double().norm()
