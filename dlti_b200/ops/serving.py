@@ -121,6 +121,19 @@ def paged_decode(q, k_cache, v_cache, block_tables, ctx_lens, H, KV, hd, scale=N
     return out
 
 
+def feed_ids(ids, src, sampled):
+    """Input ids [T] of a step: ids[t] where src[t] (int32) is -1, else sampled[src[t]], the token that the step in flight gave that
+    sequence (no host round trip between two steps)."""
+    if not _lib.use_native(ids):
+        return torch.where(src >= 0, sampled[src.clamp_min(0).long()], ids)
+    assert ids.dtype == sampled.dtype == torch.int64 and src.dtype == torch.int32
+    assert ids.is_contiguous() and src.is_contiguous() and sampled.is_contiguous() and ids.shape == src.shape
+    out = torch.empty_like(ids)
+    f = _lib.fn("dlti_feed_ids", [_V, _V, _V, _I, _V, _L, _V])
+    _lib.check(f(_lib.ptr(ids), _lib.ptr(src), _lib.ptr(sampled), sampled.numel(), _lib.ptr(out), ids.numel(), _lib.stream_ptr()), "feed_ids")
+    return out
+
+
 def sample_ref(logits, temperature, top_k, top_p, generator=None):
     """Oracle for the kept-set semantics: returns (greedy tokens, keep mask [B,V]) — the sampled
     token of the kernel must lie inside the mask; greedy rows must match exactly."""

@@ -459,11 +459,6 @@ class LLMEngine:
         step.want_lp = bool(want_lp)
         return step
 
-    def _feed(self, ids: torch.Tensor, src: torch.Tensor) -> torch.Tensor:
-        """Input ids with the rows that continue a sequence of the step in flight taken from its device-side
-        samples (no host round trip between two steps)."""
-        return torch.where(src >= 0, self._tok_dev[src.clamp_min(0).long()], ids)
-
     def _forward_step(self, step: "PackedStep"):
         """Run the forward pass of a packed step. Returns (logits [sampled rows, vocab], device views)."""
         lay = step.layout
@@ -472,12 +467,12 @@ class LLMEngine:
         v = lay.views(self._to_device(step.slot, lay.words), torch)
         if self.per_sequence:
             segs = {c: _pieces(v["segs"][a[0]:], lay.T - lay.nd, *a[1:]) for c, a in step.segs.items()}
-            logits = self.runner.forward(self._feed(v["ids"], v["src"]), v["pos"], v["slots"], num_decode=lay.nd,
+            logits = self.runner.forward(S.feed_ids(v["ids"], v["src"], self._tok_dev), v["pos"], v["slots"], num_decode=lay.nd,
                                          block_tables=v["tables"], ctx_lens=v["ctx"], cu_seqlens=v["cu"] if lay.npf else None,
                                          max_seqlen=step.max_seqlen, last_idx=v["last"] if lay.npf else None,
                                          max_ctx=self.max_model_len, state_slots=v["sslot"], row_seq=v["rseq"], segs=segs)
             return logits, v
-        logits = self.runner.forward(self._feed(v["ids"], v["src"]), v["pos"], v["slots"], num_decode=lay.nd,
+        logits = self.runner.forward(S.feed_ids(v["ids"], v["src"], self._tok_dev), v["pos"], v["slots"], num_decode=lay.nd,
                                      block_tables=v["tables"] if lay.nd else None, ctx_lens=v["ctx"] if lay.nd else None,
                                      cu_seqlens=v["cu"] if lay.npf else None, max_seqlen=step.max_seqlen,
                                      last_idx=v["last"] if lay.npf else None, max_ctx=self.max_model_len,
@@ -517,7 +512,7 @@ class LLMEngine:
                 st["sslot"].fill_(-1)
                 st["rseq"].copy_(torch.arange(bucket, device=dev))
                 kw = dict(state_slots=st["sslot"], row_seq=st["rseq"])
-            run = lambda: self.runner.forward(self._feed(st["ids"], st["src"]), st["pos"], st["slots"], num_decode=bucket,
+            run = lambda: self.runner.forward(S.feed_ids(st["ids"], st["src"], self._tok_dev), st["pos"], st["slots"], num_decode=bucket,
                                               block_tables=st["tables"], ctx_lens=st["ctx"], max_ctx=self.max_model_len, **kw)
             side = torch.cuda.Stream(device=dev)
             side.wait_stream(torch.cuda.current_stream())

@@ -347,6 +347,9 @@ int dlti_sample(const void* logits, long long ld, int batch, int V, const float*
                 const int* top_k, const float* top_p, const unsigned long long* seeds,
                 unsigned long long step, long long* out, float* out_logprob, int dtype,
                 dlti_stream_t stream);
+/* out[t] = src[t] in [0, n) ? sampled[src[t]] : ids[t]: the input ids of a step that continues the step in flight */
+int dlti_feed_ids(const long long* ids, const int* src, const long long* sampled, int n, long long* out, long long rows,
+                  dlti_stream_t stream);
 
 /* ---- Layer-stack models (models/stack.py): csrc/stack.cu, streams.cu, recurrent.cu, attention_paged.cu, latent.cu, dyt.cu, prenorm.cu,
  * conv_qkv.cu, moe.cu, delta.cu, gemm_f32.cu. Row pitches (*_ld) in

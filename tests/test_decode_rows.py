@@ -55,3 +55,12 @@ def test_recurrences_of_decode_rows(kind, heads, N, P, n, dtype):
     for x, y, tol in zip(got["cuda"], got["cpu"], (1e-5 if dtype == F32 else 4e-3, 1e-5, 1e-5)):     # fp32 sums; outputs rounded to 8 bits
         x, y = (x[live], y[live]) if x.shape[0] == n and x.dim() == 2 else (x, y)                     # rows without a slot: no result
         assert (x.double() - y.double()).norm() <= tol * y.double().norm()
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 1000])
+def test_fed_ids(n):
+    from dlti_b200.ops import serving as S
+    g = torch.Generator().manual_seed(n)
+    ids, sampled = torch.randint(0, 1 << 40, (n,), generator=g), torch.randint(0, 1 << 40, (300,), generator=g)
+    src = torch.randint(-1, 300, (n,), generator=g, dtype=torch.int32)
+    assert torch.equal(S.feed_ids(ids.cuda(), src.cuda(), sampled.cuda()).cpu(), S.feed_ids(ids, src, sampled))
