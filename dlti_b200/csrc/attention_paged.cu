@@ -393,8 +393,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, i
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ int s_slots[2][KT];
   __shared__ float s_m[4][16], s_l[4][16];
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int rep = p.H / p.G, hblocks = (rep + 15) / 16;
   const int split = blockIdx.x, b = blockIdx.z, g = blockIdx.y / hblocks, h0 = (blockIdx.y % hblocks) * 16;
   const int nh = min(16, rep - h0);
@@ -520,8 +519,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, i
 
 __global__ void __launch_bounds__(128) attn_combine_kernel(const PagedParams p, int splits, const float* __restrict__ part_o,
                                                           const float* __restrict__ part_ml) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int h = blockIdx.x, b = blockIdx.y;
   const long long base = ((long long)b * p.H + h) * splits;
   float gm = -INFINITY, gl = 0.f;

@@ -42,8 +42,7 @@ __device__ __forceinline__ Job job_of(const ConvQkv& p, int job) {
 
 template <typename T, bool ACC, int MAXE>
 __global__ void __launch_bounds__(128) conv_qkv_kernel(const ConvQkv p, int jobs) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int lane = threadIdx.x & 31, hist = p.taps - 1;
   const long long total = p.tokens * jobs;
   for (long long x = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < total; x += ((long long)gridDim.x * blockDim.x) >> 5) {
@@ -163,8 +162,7 @@ __global__ void __launch_bounds__(128) conv_qkv_vec_kernel(const ConvQkv p, int 
       for (int j = 0; j < 8; ++j) w[k][j] = k == HIST ? 1.f : 0.f;
   }
   norm_weights(p, job, e0, nw);
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long t0 = (long long)blockIdx.x * CQ_ROWS;
   const int nr = (int)min((long long)CQ_ROWS, p.tokens - t0);
   const T* src = reinterpret_cast<const T*>(p.proj) + c;
@@ -232,8 +230,7 @@ __global__ void __launch_bounds__(128) conv_qkv_decode_kernel(const ConvQkv p, i
   norm_weights(p, job, e0, nw);
   const bool conv = p.w && job.kind < 3;
   if (conv) ld8(p.w + (long long)hist * p.w_ld + c - p.oq, w);
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long t = blockIdx.x;
 #pragma unroll
   for (int j = 0; j < 8; ++j) a[j] = 0.f;
@@ -267,8 +264,7 @@ __global__ void __launch_bounds__(128) conv_qkv_decode_kernel(const ConvQkv p, i
 // the last taps - 1 inputs of every sequence become its state; entries move towards the front, so they may overwrite one another in order
 template <typename T>
 __global__ void __launch_bounds__(128) conv_state_kernel(const ConvQkv p) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int c = blockIdx.x * 128 + threadIdx.x, s = blockIdx.y, hist = p.taps - 1;
   if (c >= p.C) return;
   const int slot = p.sslot[s];

@@ -63,8 +63,7 @@ __global__ void __launch_bounds__(128) acc_add_rmsnorm_kernel(float* __restrict_
                                                               const T* __restrict__ w, T* __restrict__ y,
                                                               int d, float eps) {
   __shared__ float red[32];
-  griddep_wait();            // the GEMM that fills acc (decode steps launch these kernels as programmatic dependents)
-  griddep_launch();
+  griddep_pass(gridDim.x);   // after the GEMM that fills acc (decode steps launch these kernels as programmatic dependents)
   const long long row = blockIdx.x;
   const int nvec = d >> 3;
   int4* rr = reinterpret_cast<int4*>(res + row * d);
@@ -117,8 +116,7 @@ __global__ void __launch_bounds__(128) acc_add_rmsnorm_kernel(float* __restrict_
 template <typename T>
 __global__ void acc_swiglu_kernel(float* __restrict__ acc, T* __restrict__ h, long long rows, int ff,
                                   long long h_stride) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass(rows);
   const int vpr = ff >> 3;
   const long long total = rows * vpr;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -144,8 +142,7 @@ __global__ void acc_rope_cache_kernel(float* __restrict__ acc, T* __restrict__ q
                                       const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                       const long long* __restrict__ slots, T* __restrict__ k_cache,
                                       T* __restrict__ v_cache, long long tokens, int H, int KV, long long W) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass(tokens);
   const int heads = H + 2 * KV;
   const int vph = HD / 16;
   const long long total = tokens * heads * vph;

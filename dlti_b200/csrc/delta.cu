@@ -40,8 +40,7 @@ __device__ __forceinline__ float step_share(const DeltaParams& p, long long row,
 // token-by-token form below.
 template <typename T, int NR, int V>
 __global__ void __launch_bounds__(256, NR * V <= 32 ? 4 : 2) delta_step_kernel(const DeltaParams p, int blocks, int conv_parts) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int s = p.seq0 + blockIdx.z;
   if ((int)blockIdx.x >= blocks) {
     if (blockIdx.y == 0) conv_tail<T>(p, s, blockIdx.x - blocks, conv_parts);

@@ -67,8 +67,7 @@ __device__ __forceinline__ void x_store(float* p, const float (&f)[W]) {
 template <typename T, int W>
 __global__ void __launch_bounds__(128) tanh_embed_kernel(const long long* __restrict__ ids, const T* __restrict__ table, long long vocab,
                                                          float scale, Norm pre, float* __restrict__ x, T* __restrict__ h, long long h_ld, int d) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int c = (blockIdx.y * 128 + threadIdx.x) * W;
   if (c >= d) return;
   const long long t = blockIdx.x, id = ids[t];
@@ -101,8 +100,7 @@ template <typename T, bool ACC, int W, int ROWS>
 __global__ void __launch_bounds__(128) tanh_between_kernel(const Between p, long long tokens) {
   const int c = (blockIdx.y * 128 + threadIdx.x) * W;
   const bool on = c < p.d;
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   if (p.counts && blockIdx.x == 0 && blockIdx.y == 0)
     for (int i = threadIdx.x; i < p.ncounts; i += 128) p.counts[i] = 0;
   if (!on) return;
@@ -156,8 +154,7 @@ __global__ void __launch_bounds__(128) tanh_between_kernel(const Between p, long
 template <typename T, int W>
 __global__ void __launch_bounds__(128) tanh_rows_kernel(const float* __restrict__ x, const long long* __restrict__ idx, Norm n,
                                                         T* __restrict__ h, long long h_ld, int d) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int c = (blockIdx.y * 128 + threadIdx.x) * W;
   if (c >= d) return;
   const long long t = blockIdx.x;

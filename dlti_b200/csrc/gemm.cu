@@ -32,12 +32,15 @@ constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr int NUM_THREADS = 192;
 
-template <int BN>
+// Stages of the ring. Stream-K (decode): 120 KB in flight per SM cover HBM's latency, and what is left of the shared memory lets the
+// kernels around it start beside it; with 8 stages a step of 64 rows of 12 Llama layers of width 2048 took 856 us instead of 806
+// (6: 815; 4: 930).
+template <int BN, bool SK = false>
 struct Cfg {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128 ? 6 : 8);
+  static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128 ? (SK ? 4 : 6) : (SK ? 5 : 8));
   static constexpr int TMEM_COLS = 2 * BN;
   static constexpr int BAR_BYTES = 256;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + 1024;
@@ -155,7 +158,7 @@ gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmA,
                     const __grid_constant__ CUtensorMap tmA2,
                     const __grid_constant__ CUtensorMap tmB2,
                     const __grid_constant__ CUtensorMap tmBL, const GatherParams gp) {
-  using C_ = Cfg<BN>;
+  using C_ = Cfg<BN, SK>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t bar_base = smem_base + C_::STAGES * C_::STAGE_BYTES;
@@ -531,7 +534,7 @@ template <int BN, bool A_MN, bool B_MN, bool GATHER, bool PUSH = false, bool SK 
 int launch(const GemmParams& p, const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& a2,
            const CUtensorMap& b2, const CUtensorMap& bl, const GatherParams& gp, int grid,
            cudaStream_t stream) {
-  using C_ = Cfg<BN>;
+  using C_ = Cfg<BN, SK>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);

@@ -47,8 +47,7 @@ __device__ __forceinline__ void zero8(T* p) {
 template <bool ACC, int QP>
 __global__ void __launch_bounds__(128) latent_prep_vec_kernel(const PrepParams p, int units, int per_head) {
   using T = bf16;
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long t = blockIdx.x;
   const uint8_t* row = reinterpret_cast<const uint8_t*>(p.proj) + t * p.ld * (ACC ? 4 : sizeof(T));
   const int ps = p.pos[t], half = p.rd >> 1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -145,8 +144,7 @@ template <typename T, bool ACC>
 __global__ void __launch_bounds__(128) latent_prep_kernel(const PrepParams p) {
   __shared__ float red[32];
   extern __shared__ float cs[];                            // [rank]
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long t = blockIdx.x;
   const uint8_t* row = reinterpret_cast<const uint8_t*>(p.proj) + t * p.ld * (ACC ? 4 : sizeof(T));
   const int ps = p.pos[t], half = p.rd >> 1, npair = half + ((p.rot - p.rd + 1) >> 1), qh = p.dim + p.rot;
@@ -273,8 +271,7 @@ __global__ void __launch_bounds__(128) head_gemm_kernel(const HeadGemmParams p) 
 #pragma unroll
   for (int i = 0; i < HG_STAGES - 1; ++i)                  // weights never change: they may come before the wait
     if (i < nk) load_b(i);
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
 #pragma unroll
   for (int i = 0; i < HG_STAGES - 1; ++i) {
     if (i < nk) load_a(i);
@@ -322,8 +319,7 @@ __global__ void __launch_bounds__(128) head_gemm_kernel(const HeadGemmParams p) 
 // fp32 arithmetic, any sizes: a thread per output
 template <typename T, bool KN>
 __global__ void __launch_bounds__(128) head_gemm_any_kernel(const HeadGemmParams p) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int h = blockIdx.y, n = blockIdx.x * 128 + threadIdx.x;
   const long long t = blockIdx.z;
   if (n >= p.N) return;
@@ -395,8 +391,7 @@ __global__ void __launch_bounds__(LTHREADS) latent_decode_kernel(const LatentPar
     *err = 0;
     mbar_fence_init();
   }
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   auto wait = [&](uint32_t bar, uint32_t parity) {
     if (!mbar_try_wait(bar, parity)) {
       const long long t0 = clock64();
@@ -615,8 +610,7 @@ __global__ void __launch_bounds__(LTHREADS) latent_decode_kernel(const LatentPar
 // sum of the splits of every (row, head): four latent columns a thread
 __global__ void __launch_bounds__(128) latent_combine_kernel(const LatentParams p, int splits, const float* __restrict__ part_o,
                                                             const float* __restrict__ part_ml) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int h = blockIdx.x;
   const long long b = blockIdx.y, base = (b * p.H + h) * splits;
   float gm = -INFINITY, gl = 0.f;

@@ -163,8 +163,7 @@ __device__ __forceinline__ void route_block(const RouteParams& p, int per) {
 
 template <typename T, bool ACC, int W, int R>
 __global__ void __launch_bounds__(32 * ROUTE_WARPS) moe_route_kernel(const RouteParams p, int route_blocks, int route_per) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   if ((int)blockIdx.x < route_blocks) {
     route_block<ACC, R>(p, route_per);
     return;

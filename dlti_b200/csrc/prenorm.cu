@@ -50,8 +50,7 @@ __global__ void __launch_bounds__(THREADS) prenorm_between_kernel(const Between 
       if (c < p.d) piece_f32<W>(p.pre + c, wv[i]);
     }
   }
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long t = blockIdx.x;
   if (p.counts && t == 0)
     for (int i = threadIdx.x; i < p.ncounts; i += THREADS) p.counts[i] = 0;
@@ -152,8 +151,7 @@ template <typename T, bool ACC, int W>
 __global__ void __launch_bounds__(128) token_gate_kernel(const void* __restrict__ u, long long u_ld, const long long* __restrict__ ids,
                                                          const T* __restrict__ table, long long t_ld, long long vocab, int col, int n,
                                                          T* __restrict__ h, long long h_ld, long long tokens) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int per = n / W;
   const long long total = tokens * per;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {

@@ -45,8 +45,7 @@ __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); 
 // 8 heads of 128 x 256 (134 MB read and written): 43 -> 27 us, 5.0 TB/s. The order of all sums is that of the token-by-token form.
 template <typename T, int NR, int V, bool ML>
 __global__ void __launch_bounds__(256, NR * V <= 32 ? 4 : 2) scan_step_kernel(const ScanParams p, int blocks, int conv_parts) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int s = p.seq0 + blockIdx.z;
   if ((int)blockIdx.x >= blocks) {
     if (blockIdx.y == 0) conv_tail<T>(p, s, blockIdx.x - blocks, conv_parts);

@@ -105,8 +105,7 @@ __global__ void __launch_bounds__(128, DLTI_PAGED_MIN_CTAS) paged_decode_kernel(
     const int* __restrict__ ctx_lens, int block_size, int H, int KV, float scale_log2,
     float* __restrict__ part_o, float* __restrict__ part_ml, int splits, T* __restrict__ out,
     long long out_stride) {
-  griddep_wait();            // q and this step's K/V rows come from the kernel before (see dlti_launch_pdl)
-  griddep_launch();
+  griddep_pass(gridDim.z);   // q and this step's K/V rows come from the kernel before (see dlti_launch_pdl)
   const int split = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int ctx = ctx_lens[b];
   const int kvh = h / (H / KV);
@@ -250,8 +249,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) paged_combine_kernel(const float* __restrict__ part_o,
                                                            const float* __restrict__ part_ml, int splits,
                                                            T* __restrict__ out, long long out_stride, int H) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass(gridDim.y);
   const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
   const long long base = ((long long)b * H + h) * splits;
   float gm = -INFINITY;
@@ -438,8 +436,7 @@ inline int grid_for(long long total, int block) {
 __global__ void __launch_bounds__(128) feed_ids_kernel(const long long* __restrict__ ids, const int* __restrict__ src,
                                                        const long long* __restrict__ sampled, int n, long long* __restrict__ out,
                                                        long long rows) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long t = (long long)blockIdx.x * 128 + threadIdx.x;
   if (t >= rows) return;
   const int s = src[t];

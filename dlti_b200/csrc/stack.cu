@@ -10,8 +10,7 @@ namespace {
 template <typename T>
 __global__ void embed_rows_kernel(const long long* __restrict__ ids, const T* __restrict__ table, float* __restrict__ x,
                                   T* __restrict__ xa, long long xa_ld, long long tokens, int d, long long vocab) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long total = tokens * d;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long t = i / d;
@@ -25,8 +24,7 @@ __global__ void embed_rows_kernel(const long long* __restrict__ ids, const T* __
 
 // out = scale * acc (fp32), with cap > 0: cap * tanh(scale * acc / cap); clear: acc = 0 (otherwise out may be acc)
 __global__ void take_rows_kernel(float* acc, float* out, float scale, float cap, int clear, long long vec) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vec; i += (long long)gridDim.x * blockDim.x) {
     float4 v = reinterpret_cast<float4*>(acc)[i];
     if (clear) reinterpret_cast<float4*>(acc)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -43,8 +41,7 @@ __global__ void __launch_bounds__(PN_THREADS) post_norm_add_kernel(const void* _
                                                                   const float* __restrict__ w, T* __restrict__ xa,
                                                                   long long xa_ld, int d, float eps, float one) {
   __shared__ float red[32];
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long row = blockIdx.x;
   const void* yr = reinterpret_cast<const uint8_t*>(y) + row * y_ld * (ACC ? 4 : sizeof(T));
   float* xr = x + row * d;
@@ -89,8 +86,7 @@ __global__ void __launch_bounds__(128) post_norm_add_vec_kernel(const void* __re
     const int v = threadIdx.x + i * 128;
     if (v < vec) ld8(w + v * 8, wv[i]);
   }
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long row = blockIdx.x;
   const void* yr = reinterpret_cast<const uint8_t*>(y) + row * y_ld * (ACC ? 4 : sizeof(T));
   float* xr = x + row * d;
@@ -129,8 +125,7 @@ __global__ void __launch_bounds__(PN_THREADS) rms_rows_kernel(const float* __res
                                                              const float* __restrict__ w, T* __restrict__ out,
                                                              long long out_ld, int d, float eps, float one) {
   __shared__ float red[32];
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const float* xr = x + (idx ? idx[blockIdx.x] : (long long)blockIdx.x) * d;
   float ss = 0.f;
   for (int c = threadIdx.x; c < d; c += PN_THREADS) ss += xr[c] * xr[c];
@@ -143,8 +138,7 @@ __global__ void __launch_bounds__(PN_THREADS) rms_rows_kernel(const float* __res
 // h = relu(u)^2, columns in pairs (row pitches are even)
 template <typename T, bool ACC>
 __global__ void relu2_kernel(const void* __restrict__ u, long long u_ld, T* __restrict__ h, long long h_ld, long long rows, int ff) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int pairs = (ff + 1) >> 1;
   const long long total = rows * pairs;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -166,8 +160,7 @@ __global__ void relu2_kernel(const void* __restrict__ u, long long u_ld, T* __re
 // the same, 8 columns per thread (16-bit, both pitches and ff multiples of 8)
 template <typename T, bool ACC>
 __global__ void relu2_vec_kernel(const void* __restrict__ u, long long u_ld, T* __restrict__ h, long long h_ld, long long rows, int ff) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int vec = ff >> 3;
   const long long total = rows * vec;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -196,8 +189,7 @@ __global__ void __launch_bounds__(256) gated_norm_kernel(const T* __restrict__ y
                                                          long long o_ld, int n, int groups, float eps) {
   __shared__ float red[32];
   extern __shared__ float row_s[];          // the gated row (GATE_FIRST) or the gate factors
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long t = blockIdx.x;
   const T* yr = y + t * y_ld;
   const void* gr = reinterpret_cast<const uint8_t*>(gate) + t * g_ld * (ACC ? 4 : sizeof(T));
@@ -241,8 +233,7 @@ __global__ void __launch_bounds__(512) gated_norm_vec_kernel(const T* __restrict
                                                              long long g_ld, const float* __restrict__ w, T* __restrict__ out,
                                                              long long o_ld, int gs, float eps) {
   __shared__ float red[32];
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long t = blockIdx.x;
   const int c0 = blockIdx.y * gs, vec = gs >> 3;
   const T* yr = y + t * y_ld;
@@ -287,8 +278,7 @@ template <typename T, int GATE, bool ACC, int VPT, int LPG>
 __global__ void __launch_bounds__(256) gated_norm_warp_kernel(const T* __restrict__ y, long long y_ld, const void* __restrict__ gate,
                                                               long long g_ld, const float* __restrict__ w, T* __restrict__ out,
                                                               long long o_ld, int gs, int groups, long long total, float eps) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long x0 = ((long long)blockIdx.x * 256 + threadIdx.x) / LPG, x = min(x0, total - 1);       // whole warps take part in the sums
   const long long t = x / groups;
   const int c0 = (int)(x - t * groups) * gs, vec = x0 < total ? gs >> 3 : 0, lane = threadIdx.x % LPG;
@@ -347,8 +337,7 @@ __device__ __forceinline__ long long q_row(const QkvParams& p, long long t) {
 constexpr int QKV_MAXP = 8;               // pairs per lane: heads of up to 512
 template <typename T, bool ACC>
 __global__ void __launch_bounds__(256) qk_norm_rope_cache_kernel(const QkvParams p) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const bool own = p.ok >= 0, copy_kv = !own && p.kp;
   const int kvjobs = (own || copy_kv) ? 2 * p.G : 0;
   const int jobs = p.H + kvjobs + (p.og >= 0 ? 1 : 0);
@@ -444,8 +433,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_cache_kernel(const QkvParams
 template <typename T, bool ACC, int LPH, int JPW>
 __global__ void __launch_bounds__(128) qk_norm_rope_cache_vec_kernel(const QkvParams p, int jobs, int kvjobs) {
   constexpr int HPW = 32 / LPH, HD = 8 * LPH;
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int lane = threadIdx.x & 31, sub = lane % LPH, e0 = sub * 8, half = p.rot >> 1;
   const long long t = blockIdx.x;
   const int job0 = (blockIdx.y * 4 + (threadIdx.x >> 5)) * (HPW * JPW);
@@ -547,8 +535,7 @@ template <typename T, bool ACC, int W>
 __global__ void __launch_bounds__(256) qkv_rows_kernel(const QkvRowParams p) {
   __shared__ float red[32];
   extern __shared__ __align__(16) float row_q[];           // q, then k
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long t = blockIdx.x;
   const uint8_t* row = reinterpret_cast<const uint8_t*>(p.proj) + t * p.ld * (ACC ? 4 : sizeof(T));
   const long long slot = p.slots[t];
@@ -609,8 +596,7 @@ __global__ void __launch_bounds__(256) qkv_rows_kernel(const QkvRowParams p) {
 template <typename T, bool ACC, int VPT, int THREADS>
 __global__ void __launch_bounds__(THREADS) qkv_rows_vec_kernel(const QkvRowParams p) {
   __shared__ float2 red[THREADS / 32];
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long t = blockIdx.x;
   const uint8_t* row = reinterpret_cast<const uint8_t*>(p.proj) + t * p.ld * (ACC ? 4 : sizeof(T));
   const long long slot = p.slots[t];
@@ -701,8 +687,7 @@ struct ConvParams {
 };
 template <typename T>
 __global__ void __launch_bounds__(256) short_conv_kernel(const ConvParams p) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int pairs = (p.C + 1) >> 1;
   const long long total = p.rows * pairs;
   const T* src = reinterpret_cast<const T*>(p.src);
@@ -743,8 +728,7 @@ __global__ void __launch_bounds__(256) short_conv_kernel(const ConvParams p) {
 constexpr int CONV_ROWS = 8;
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128) short_conv_vec_kernel(const ConvParams p) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int vec = p.C >> 3, cv = blockIdx.y * 128 + threadIdx.x;
   if (cv >= vec) return;
   const int c = cv * 8;
@@ -817,8 +801,7 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(const ConvParams p)
 // decode rows only: the projection comes as the decode GEMM's accumulator
 template <typename T>
 __global__ void __launch_bounds__(256) short_conv_acc_kernel(const ConvParams p) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int pairs = (p.raw_n + 1) >> 1;
   const long long total = p.rows * pairs;
   const T* state = reinterpret_cast<const T*>(p.state);
@@ -855,8 +838,7 @@ __global__ void __launch_bounds__(256) short_conv_acc_kernel(const ConvParams p)
 // the same, 8 columns per thread (C, col and every pitch multiples of 8)
 template <typename T>
 __global__ void __launch_bounds__(128) short_conv_acc_vec_kernel(const ConvParams p) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int col = (blockIdx.y * 128 + threadIdx.x) * 8;
   if (col >= p.raw_n) return;
   const long long t = blockIdx.x;

@@ -57,8 +57,7 @@ __global__ void __launch_bounds__(512) hyper_vec_kernel(const HyperParams p) {
 #pragma unroll
     for (int t = 0; t < S; ++t) mix[s][t] = p.y ? p.mix[s * S + t] : 0.f;
   }
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long row = p.idx ? p.idx[blockIdx.x] : (long long)blockIdx.x;
   float* xr = p.x + row * S * p.d;
   const void* yr = reinterpret_cast<const uint8_t*>(p.y) + row * p.y_ld * (ACC ? 4 : sizeof(T));
@@ -129,8 +128,7 @@ template <typename T, bool ACC>
 __global__ void __launch_bounds__(256) hyper_kernel(const HyperParams p) {
   __shared__ float red[32];
   extern __shared__ float u[];                             // [d]; a thread only touches its own channels
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int S = p.S;
   const long long row = p.idx ? p.idx[blockIdx.x] : (long long)blockIdx.x;
   float* xr = p.x + row * S * p.d;
@@ -209,8 +207,7 @@ int launch_hyper(const HyperParams& p, long long rows, cudaStream_t st) {
 template <typename T>
 __global__ void embed_streams_kernel(const long long* __restrict__ ids, const T* __restrict__ table, float* __restrict__ x, long long tokens,
                                      int S, int d, long long vocab, float scale) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long total = tokens * d;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long t = i / d;
@@ -232,8 +229,7 @@ struct CanonParams {
 };
 template <typename T>
 __global__ void __launch_bounds__(128) canon_kernel(const CanonParams p) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int c = blockIdx.y * 128 + threadIdx.x, s = p.seq0 + blockIdx.z, hist = p.taps - 1;
   long long row0;
   int n, start;
@@ -263,8 +259,7 @@ __global__ void __launch_bounds__(128) canon_kernel(const CanonParams p) {
 constexpr int CANON_ROWS = 8;
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128) canon_vec_kernel(const CanonParams p) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int cv = blockIdx.y * 128 + threadIdx.x, s = p.seq0 + blockIdx.z;
   long long row0;
   int n, start;
@@ -336,8 +331,7 @@ __global__ void __launch_bounds__(NT) poly_norm_vec_kernel(const void* __restric
                                                             T* __restrict__ out, long long o_ld, int n, float eps) {
   __shared__ float red[96];
   const float a = coef[0], b = coef[1], c = coef[2], e = coef[3];
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long row = blockIdx.x;
   const void* zr = reinterpret_cast<const uint8_t*>(z) + row * z_ld * (ACC ? 4 : sizeof(T));
   const int vec = n >> 3;
@@ -374,8 +368,7 @@ __global__ void __launch_bounds__(256) poly_norm_kernel(const void* __restrict__
                                                         T* __restrict__ out, long long o_ld, int n, float eps) {
   __shared__ float red[96];
   extern __shared__ float row_s[];
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const long long row = blockIdx.x;
   const void* zr = reinterpret_cast<const uint8_t*>(z) + row * z_ld * (ACC ? 4 : sizeof(T));
   float3 s = make_float3(0.f, 0.f, 0.f);
@@ -398,8 +391,7 @@ __global__ void __launch_bounds__(256) poly_norm_kernel(const void* __restrict__
 template <typename T>
 __global__ void split_rows_kernel(float* __restrict__ acc, T* __restrict__ out, long long o_ld, float* __restrict__ tail, long long t_ld,
                                   long long rows, int n, int split) {
-  griddep_wait();
-  griddep_launch();
+  griddep_pass();
   const int vec = n >> 3;
   const long long total = rows * vec;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
