@@ -32,6 +32,9 @@ struct ScanParams {
   const float *gates, *gate_b; long long g_ld;
   float cap, q_scale;
   float* vec;
+  // chunked form in segments: tokens of a segment (a multiple of 64), segments of the longest sequence, see SegEntry
+  int seg_len, segs;
+  float* seg_ws;
 };
 
 // log gates of an mLSTM head: cap tanh(z / cap), for the forget gate the logarithm of its sigmoid
@@ -380,6 +383,14 @@ int launch_scan(const ScanParams& p, int nseq, cudaStream_t st) {
 // of the old state 2^(m - A_t): the same products with -A in the place of L and 2^a in that of the step sizes. n is one more
 // column of the state product (its operand: the scaling factors themselves, hi in column 0 and lo in column 1), and
 // n . q the row sums of the bracketed weights plus one more column of S^T q.
+//
+// One sequence gives only heads * P / 32 CTAs, each a chain of n / 64 chunks. Where that leaves SMs without work, the sequence is
+// cut into segments of whole chunks: a first launch (SEG_STATE) runs the state half alone over every segment but the last, from
+// zero (the first one from the carried state), and leaves S, the segment's decay and for an mLSTM n and m in a SegEntry; the second
+// (SEG_FULL) starts every segment from the entries before it, folded in order. The state half is under half of the work of a chunk.
+// One prompt of 8192 tokens: 64 heads of 128 x 64 (128 CTAs, 2 segments) and 16 heads of 128 x 128 (64 CTAs, 4 segments) took 408 us on
+// average, now 270 in both launches together.
+constexpr int WHOLE = 0, SEG_STATE = 1, SEG_FULL = 2;
 constexpr int CQ = 64, CP = 32, CPP = CP + 8;
 template <int NT>
 struct ChunkSmem {
@@ -392,13 +403,17 @@ struct ChunkVec {                                                // one chunk's 
   float *L, *step, *E, *F;                                       // L; d; 2^(L_63 - L_s) d; 2^(L_e - L_s) d, e = end of s's 16-block
   float *floor, *m;                                              // mLSTM: exp(-m_t); m before the chunk. L = -A, step = a
 };
-template <int NT, bool ML>
+// What a segment leaves for those after it, fp32: S [NT][32], n [NT], {log2 of its decay, m in log2}. The entry of a sequence's last
+// segment holds the state that the sequence brought: nothing may read p.state in the second launch, which renews it.
+template <int NT>
+struct SegEntry { static constexpr int N = NT * CP, LOG = N + NT, FLOATS = LOG + 4; };
+template <int NT, bool ML, int MODE>
 __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(const ScanParams p, int slices, int conv_parts) {
   using L = ChunkSmem<NT>;
   using bf16 = __nv_bfloat16;
-  const int s = p.seq0 + blockIdx.z;
+  const int sq = MODE == WHOLE ? blockIdx.z : blockIdx.z / p.segs, seg = MODE == WHOLE ? 0 : blockIdx.z - sq * p.segs, s = p.seq0 + sq;
   if ((int)blockIdx.x >= slices) {
-    if (blockIdx.y == 0) conv_tail<bf16>(p, s, blockIdx.x - slices, conv_parts);
+    if (blockIdx.y == 0 && seg == 0) conv_tail<bf16>(p, s, blockIdx.x - slices, conv_parts);
     return;
   }
   extern __shared__ __align__(128) uint8_t smem[];
@@ -409,6 +424,10 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
   const int h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = blockIdx.x * CP, ncol = min(CP, p.P - c0), grp = h / p.rep;
   const int slot = p.sslot[s];
+  const int last_seg = MODE == WHOLE ? 0 : min((n - 1) / p.seg_len, p.segs - 1);       // the tokens [tb, te) are this CTA's
+  if (MODE != WHOLE && (n <= 0 || seg > last_seg || (MODE == SEG_STATE && seg == last_seg))) return;
+  const int tb = MODE == WHOLE ? 0 : seg * p.seg_len, te = seg == last_seg ? n : tb + p.seg_len;
+  auto entry = [&](int i) { return p.seg_ws + ((((long long)sq * p.segs + i) * p.heads + h) * slices + blockIdx.x) * SegEntry<NT>::FLOATS; };
   const bf16* q = reinterpret_cast<const bf16*>(p.q) + row0 * p.q_ld + (long long)grp * p.N;
   const bf16* k = reinterpret_cast<const bf16*>(p.k) + row0 * p.k_ld + (long long)grp * p.N;
   const bf16* v = reinterpret_cast<const bf16*>(p.v) + row0 * p.v_ld + (long long)h * p.P + c0;
@@ -428,7 +447,7 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
 #pragma unroll
     for (int i = 0; i < CQ / STEP; ++i) {
       const bool ok = cok && t0 + r0 + i * STEP < n;
-      cp_async16(dst + i * STEP * L::NP * 2, ok ? qp : q, ok);
+      if (MODE != SEG_STATE) cp_async16(dst + i * STEP * L::NP * 2, ok ? qp : q, ok);
       cp_async16(dst + i * STEP * L::NP * 2 + L::QK, ok ? kp : k, ok);
       qp += STEP * p.q_ld;
       kp += STEP * p.k_ld;
@@ -438,16 +457,149 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
     cp_async16(base + 2 * L::QK + (r * CPP + cv * 8) * 2, ok ? v + (t0 + r) * p.v_ld + cv * 8 : v, ok);
     cp_async_commit();
   };
-  load(0, 0);
+  load(0, tb);
 
+  const bool have = slot >= 0 && start > 0;
+  constexpr float LOG2E = 1.4426950408889634f;
+  const float eA = ML || p.decay ? 0.f : expf(p.A_log[h]) * LOG2E;
+  const float la_c = !ML && p.decay ? fmaxf(logf(p.decay[h]), -80.f) * LOG2E : 0.f;
+  const float bias = ML ? p.gate_b[h] : (p.decay ? 0.f : p.dt_bias[h]);
+  const float bias_f = ML ? p.gate_b[p.heads + h] : 0.f;
+  float* vecs = ML ? p.vec + (((long long)(slot < 0 ? 0 : slot) * p.heads + h) * slices + blockIdx.x) * (p.N + 1) : nullptr;
+  float logs = 0.f;                                              // warp PREP: log2 of the decay of the chunks prepared so far
+  float m = 0.f;                                                 // warp PREP, mLSTM: log2 of the running maximum
+  // warp PREP: step sizes and decays of the chunk at t0, two consecutive tokens a lane
+  auto raw_dt = [&](int t0, float (&d)[4]) {                     // mLSTM: input gates, then forget gates
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const int t = t0 + 2 * lane + y;
+      if constexpr (ML) {
+        d[y] = t < n ? p.gates[(row0 + t) * p.g_ld + h] + bias : 0.f;
+        d[2 + y] = t < n ? p.gates[(row0 + t) * p.g_ld + p.heads + h] + bias_f : 0.f;
+      } else
+      d[y] = (!p.decay && t < n) ? __bfloat162float(reinterpret_cast<const bf16*>(p.dt)[(row0 + t) * p.dt_ld + h]) + bias : 0.f;
+    }
+  };
+  auto prepare_ml = [&](int i, int t0, const float (&d)[4]) {
+    float f[2], a[2];
+#pragma unroll
+    for (int y = 0; y < 2; ++y) f[y] = t0 + 2 * lane + y < n ? log_forget_gate(d[2 + y], p.cap) * LOG2E : 0.f;
+    f[1] += f[0];
+    float x = f[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    const float F1 = x, F0 = x - f[1] + f[0];
+#pragma unroll
+    for (int y = 0; y < 2; ++y) a[y] = t0 + 2 * lane + y < n ? log_in_gate(d[y], p.cap) * LOG2E - (y ? F1 : F0) : -INFINITY;
+    x = fmaxf(a[0], a[1]);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x = fmaxf(x, y);
+    }
+    float before = __shfl_up_sync(0xffffffffu, x, 1);
+    before = lane == 0 ? m : fmaxf(m, before);
+    const float A0 = fmaxf(before, a[0]), A1 = fmaxf(A0, a[1]);
+    const float last = __shfl_sync(0xffffffffu, A1, 31), Ae = __shfl_sync(0xffffffffu, A1, lane | 7);
+    const ChunkVec cv = vec(i);
+    *reinterpret_cast<float2*>(cv.L + 2 * lane) = make_float2(-A0, -A1);
+    *reinterpret_cast<float2*>(cv.step + 2 * lane) = make_float2(a[0], a[1]);
+    *reinterpret_cast<float2*>(cv.E + 2 * lane) = make_float2(ex2(a[0] - last), ex2(a[1] - last));
+    *reinterpret_cast<float2*>(cv.F + 2 * lane) = make_float2(ex2(a[0] - Ae), ex2(a[1] - Ae));
+    *reinterpret_cast<float2*>(cv.floor + 2 * lane) = make_float2(ex2(-(F0 + A0)), ex2(-(F1 + A1)));
+    if (lane == 0) *cv.m = m;
+    const float F = __shfl_sync(0xffffffffu, F1, 31);
+    logs += F;
+    m = F + last;
+  };
+  auto prepare = [&](int i, int t0, const float (&d)[4]) {
+    float step[2], l[2];
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const bool ok = t0 + 2 * lane + y < n;
+      step[y] = !ok ? 0.f : (p.decay ? 1.f : softplus_f(d[y]));
+      l[y] = !ok ? 0.f : (p.decay ? la_c : -eA * step[y]);
+    }
+    l[1] += l[0];
+    float x = l[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    const float before = x - l[1];
+    const float total = __shfl_sync(0xffffffffu, x, 31);
+    logs += total;
+    const float le = __shfl_sync(0xffffffffu, x, lane | 7);      // end of this 16-token block
+    const float l0 = before + l[0], l1 = x;
+    const ChunkVec cv = vec(i);
+    *reinterpret_cast<float2*>(cv.L + 2 * lane) = make_float2(l0, l1);
+    *reinterpret_cast<float2*>(cv.step + 2 * lane) = make_float2(step[0], step[1]);
+    *reinterpret_cast<float2*>(cv.E + 2 * lane) = make_float2(ex2(total - l0) * step[0], ex2(total - l1) * step[1]);
+    *reinterpret_cast<float2*>(cv.F + 2 * lane) = make_float2(ex2(le - l0) * step[0], ex2(le - l1) * step[1]);
+  };
+  auto fold_m = [&](int i, float& m, float& keep, float& gain) {  // the entry of segment i behind a maximum m: factors of old and new
+    const float *e = entry(i) + SegEntry<NT>::LOG, F = e[0], mi = e[1], x = fmaxf(F + m, mi);
+    keep = ex2(F + m - x);
+    gain = ex2(mi - x);
+    m = x;
+  };
+  float d[4] = {0.f, 0.f, 0.f, 0.f};
+  // the warp that prepares the vectors: see above; the gates of an mLSTM are more than the slack of warp 0
+  constexpr int PREP = ML && MODE != SEG_STATE ? 4 : 0;
+  if (warp == PREP) {
+    if constexpr (ML) {
+      if (MODE == SEG_FULL && seg > 0) {
+        m = entry(0)[SegEntry<NT>::LOG + 1];
+        float keep, gain;
+        for (int i = 1; i < seg; ++i) fold_m(i, m, keep, gain);
+      } else if (MODE == SEG_FULL && last_seg > 0) {
+        m = entry(last_seg)[SegEntry<NT>::LOG + 1];
+      } else if (MODE == SEG_STATE && seg > 0) {
+        m = -INFINITY;
+      } else if (have) {
+        m = vecs[p.N] * LOG2E;
+      }
+      if (MODE == SEG_STATE && seg == 0 && lane == 0) entry(last_seg)[SegEntry<NT>::LOG + 1] = m;
+    }
+    raw_dt(tb, d);
+    if constexpr (ML) prepare_ml(0, tb, d);
+    else prepare(0, tb, d);
+    raw_dt(tb + CQ, d);
+  }
+  auto prepare_next = [&](int it, int t0) {                      // the vectors of the chunk after the one at t0
+    if (warp != PREP || t0 + CQ >= te) return;
+    if constexpr (ML) prepare_ml(it + 1, t0 + CQ, d);
+    else prepare(it + 1, t0 + CQ, d);
+    raw_dt(t0 + 2 * CQ, d);
+  };
+
+  if (MODE == SEG_STATE && warp < 4) {
+    int it = 0;
+    for (int t0 = tb; t0 < te; t0 += CQ, ++it) {
+      cp_async_wait<0>();
+      __syncthreads();
+      if (t0 + CQ < te) load((it + 1) & 1, t0 + CQ);
+      prepare_next(it, t0);
+    }
+    if (warp == 0 && lane == 0) {
+      float* e = entry(seg) + SegEntry<NT>::LOG;
+      e[0] = logs;
+      e[1] = m;
+    }
+    return;
+  }
   if (warp < 4) {
     // ---- outputs of 16 tokens per chunk ----
     const int scol = (lane & 3) * 2, tr = warp * 16 + (lane >> 2);
     int it = 0;
-    for (int t0 = 0; t0 < n; t0 += CQ, ++it) {
+    for (int t0 = tb; t0 < te; t0 += CQ, ++it) {
       cp_async_wait<0>();
       __syncthreads();                                           // tile, vectors and S operand of this chunk are there
-      if (t0 + CQ < n) load((it + 1) & 1, t0 + CQ);
+      if (t0 + CQ < te) load((it + 1) & 1, t0 + CQ);
       const uint32_t base = sb + (it & 1) * L::STAGE;
       const ChunkVec cv = vec(it);
       uint32_t qf[NT / 16][4];
@@ -567,94 +719,17 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
           }
         }
       }
+      prepare_next(it, t0);
     }
     return;
   }
 
   // ---- state ----
   const int sw = warp - 4;
-  constexpr float LOG2E = 1.4426950408889634f;
-  const float eA = ML || p.decay ? 0.f : expf(p.A_log[h]) * LOG2E;
-  const float la_c = !ML && p.decay ? fmaxf(logf(p.decay[h]), -80.f) * LOG2E : 0.f;
-  const float bias = ML ? p.gate_b[h] : (p.decay ? 0.f : p.dt_bias[h]);
-  const float bias_f = ML ? p.gate_b[p.heads + h] : 0.f;
-  float* vecs = ML ? p.vec + (((long long)(slot < 0 ? 0 : slot) * p.heads + h) * slices + blockIdx.x) * (p.N + 1) : nullptr;
-  float m = 0.f;                                                 // warp 4, mLSTM: log2 of the running maximum
-  // warp 4: step sizes and decays of the chunk at t0, two consecutive tokens a lane
-  auto raw_dt = [&](int t0, float (&d)[4]) {                     // mLSTM: input gates, then forget gates
-#pragma unroll
-    for (int y = 0; y < 2; ++y) {
-      const int t = t0 + 2 * lane + y;
-      if constexpr (ML) {
-        d[y] = t < n ? p.gates[(row0 + t) * p.g_ld + h] + bias : 0.f;
-        d[2 + y] = t < n ? p.gates[(row0 + t) * p.g_ld + p.heads + h] + bias_f : 0.f;
-      } else
-      d[y] = (!p.decay && t < n) ? __bfloat162float(reinterpret_cast<const bf16*>(p.dt)[(row0 + t) * p.dt_ld + h]) + bias : 0.f;
-    }
-  };
-  auto prepare_ml = [&](int i, int t0, const float (&d)[4]) {
-    float f[2], a[2];
-#pragma unroll
-    for (int y = 0; y < 2; ++y) f[y] = t0 + 2 * lane + y < n ? log_forget_gate(d[2 + y], p.cap) * LOG2E : 0.f;
-    f[1] += f[0];
-    float x = f[1];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    const float F1 = x, F0 = x - f[1] + f[0];
-#pragma unroll
-    for (int y = 0; y < 2; ++y) a[y] = t0 + 2 * lane + y < n ? log_in_gate(d[y], p.cap) * LOG2E - (y ? F1 : F0) : -INFINITY;
-    x = fmaxf(a[0], a[1]);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x = fmaxf(x, y);
-    }
-    float before = __shfl_up_sync(0xffffffffu, x, 1);
-    before = lane == 0 ? m : fmaxf(m, before);
-    const float A0 = fmaxf(before, a[0]), A1 = fmaxf(A0, a[1]);
-    const float last = __shfl_sync(0xffffffffu, A1, 31), Ae = __shfl_sync(0xffffffffu, A1, lane | 7);
-    const ChunkVec cv = vec(i);
-    *reinterpret_cast<float2*>(cv.L + 2 * lane) = make_float2(-A0, -A1);
-    *reinterpret_cast<float2*>(cv.step + 2 * lane) = make_float2(a[0], a[1]);
-    *reinterpret_cast<float2*>(cv.E + 2 * lane) = make_float2(ex2(a[0] - last), ex2(a[1] - last));
-    *reinterpret_cast<float2*>(cv.F + 2 * lane) = make_float2(ex2(a[0] - Ae), ex2(a[1] - Ae));
-    *reinterpret_cast<float2*>(cv.floor + 2 * lane) = make_float2(ex2(-(F0 + A0)), ex2(-(F1 + A1)));
-    if (lane == 0) *cv.m = m;
-    m = __shfl_sync(0xffffffffu, F1, 31) + last;
-  };
-  auto prepare = [&](int i, int t0, const float (&d)[4]) {
-    float step[2], l[2];
-#pragma unroll
-    for (int y = 0; y < 2; ++y) {
-      const bool ok = t0 + 2 * lane + y < n;
-      step[y] = !ok ? 0.f : (p.decay ? 1.f : softplus_f(d[y]));
-      l[y] = !ok ? 0.f : (p.decay ? la_c : -eA * step[y]);
-    }
-    l[1] += l[0];
-    float x = l[1];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    const float before = x - l[1];
-    const float total = __shfl_sync(0xffffffffu, x, 31);
-    const float le = __shfl_sync(0xffffffffu, x, lane | 7);      // end of this 16-token block
-    const float l0 = before + l[0], l1 = x;
-    const ChunkVec cv = vec(i);
-    *reinterpret_cast<float2*>(cv.L + 2 * lane) = make_float2(l0, l1);
-    *reinterpret_cast<float2*>(cv.step + 2 * lane) = make_float2(step[0], step[1]);
-    *reinterpret_cast<float2*>(cv.E + 2 * lane) = make_float2(ex2(total - l0) * step[0], ex2(total - l1) * step[1]);
-    *reinterpret_cast<float2*>(cv.F + 2 * lane) = make_float2(ex2(le - l0) * step[0], ex2(le - l1) * step[1]);
-  };
   constexpr int MT = NT / 64;                                    // 16-row state tiles of a warp
   float S[MT][CP / 8][4];
   float* st = p.state + (((long long)(slot < 0 ? 0 : slot) * p.heads + h) * p.N) * p.P + c0;
   const int srow = sw * (NT / 4) + (lane >> 2), scol = (lane & 3) * 2;
-  const bool have = slot >= 0 && start > 0;
   float ns[ML ? MT : 1][4];                                      // mLSTM: columns 0 (from hi) and 1 (from lo) in lanes 4 r; n is their sum
   auto publish = [&]() {                                         // S as hi / lo operands
     if constexpr (ML) {
@@ -683,41 +758,51 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
           *reinterpret_cast<uint32_t*>(smem + L::S + NT * CPP * 2 + off) = lo;
         }
   };
-  float d[4] = {0.f, 0.f, 0.f, 0.f};
-  if constexpr (ML) {
-    if (have) m = vecs[p.N] * LOG2E;
+  // the state before the segment: carried, from zero, or the entries of the segments before it
+  auto each = [&](auto f) {
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
-      for (int y = 0; y < 2; ++y) {
-        const int r = srow + i * 16 + 8 * y;
-        ns[i][2 * y] = have && (lane & 3) == 0 && r < p.N ? vecs[r] : 0.f;
-        ns[i][2 * y + 1] = 0.f;
-      }
+      for (int j = 0; j < CP / 8; ++j)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) f(S[i][j][x], srow + i * 16 + 8 * (x >> 1), j * 8 + scol + (x & 1));
+  };
+  auto each_n = [&](auto f) {
+    if constexpr (ML)
+#pragma unroll
+      for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) f(ns[i][2 * y], ns[i][2 * y + 1], srow + i * 16 + 8 * y);
+  };
+  if (MODE == SEG_FULL && last_seg > 0) {
+    const float* e = entry(seg > 0 ? 0 : last_seg);
+    each([&](float& x, int r, int c) { x = e[r * CP + c]; });
+    each_n([&](float& a, float& b, int r) { a = (lane & 3) == 0 ? e[SegEntry<NT>::N + r] : 0.f; b = 0.f; });
+    float mm = ML && seg > 0 ? e[SegEntry<NT>::LOG + 1] : 0.f;
+    for (int i = 1; i < seg; ++i) {
+      const float* ei = entry(i);
+      float keep, gain = 1.f;
+      if constexpr (ML) fold_m(i, mm, keep, gain);
+      else keep = ex2(ei[SegEntry<NT>::LOG]);
+      each([&](float& x, int r, int c) { x = fmaf(keep, x, gain * ei[r * CP + c]); });
+      each_n([&](float& a, float&, int r) { if ((lane & 3) == 0) a = fmaf(keep, a, gain * ei[SegEntry<NT>::N + r]); });
+    }
+  } else {
+    const bool carried = have && (MODE != SEG_STATE || seg == 0);
+    each([&](float& x, int r, int c) { x = carried && r < p.N && c < ncol ? st[(long long)r * p.P + c] : 0.f; });
+    each_n([&](float& a, float& b, int r) { a = carried && (lane & 3) == 0 && r < p.N ? vecs[r] : 0.f; b = 0.f; });
+    if (MODE == SEG_STATE && seg == 0) {
+      float* e = entry(last_seg);
+      each([&](float& x, int r, int c) { e[r * CP + c] = x; });
+      each_n([&](float& a, float&, int r) { if ((lane & 3) == 0) e[SegEntry<NT>::N + r] = a; });
+    }
   }
-  if (sw == 0) {
-    raw_dt(0, d);
-    if constexpr (ML) prepare_ml(0, 0, d);
-    else prepare(0, 0, d);
-    raw_dt(CQ, d);
-  }
-#pragma unroll
-  for (int i = 0; i < MT; ++i)
-#pragma unroll
-    for (int j = 0; j < CP / 8; ++j)
-#pragma unroll
-      for (int y = 0; y < 2; ++y) {
-        const int r = srow + i * 16 + 8 * y, c = j * 8 + scol;
-        const bool ok = have && r < p.N && c < ncol;             // ncol is a multiple of 8
-        S[i][j][2 * y] = ok ? st[(long long)r * p.P + c] : 0.f;
-        S[i][j][2 * y + 1] = ok ? st[(long long)r * p.P + c + 1] : 0.f;
-      }
-  publish();
+  if (MODE != SEG_STATE) publish();
   int it = 0;
-  for (int t0 = 0; t0 < n; t0 += CQ, ++it) {
+  for (int t0 = tb; t0 < te; t0 += CQ, ++it) {
     cp_async_wait<0>();
     __syncthreads();
-    if (t0 + CQ < n) load((it + 1) & 1, t0 + CQ);
+    if (t0 + CQ < te) load((it + 1) & 1, t0 + CQ);
     const uint32_t base = sb + (it & 1) * L::STAGE;
     const ChunkVec cv = vec(it);
     const bf16* sv = reinterpret_cast<const bf16*>(smem + (it & 1) * L::STAGE + 2 * L::QK);
@@ -774,15 +859,16 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
         if constexpr (ML) mma_bf16(ns[i], a, e0, e1);
       }
     }
-    if (sw == 0 && t0 + CQ < n) {
-      if constexpr (ML) prepare_ml(it + 1, t0 + CQ, d);
-      else prepare(it + 1, t0 + CQ, d);
-      raw_dt(t0 + 2 * CQ, d);
-    }
+    if (MODE == SEG_STATE) continue;
+    prepare_next(it, t0);
     asm volatile("bar.sync 2, 256;" ::: "memory");               // warps 0-3 have read the old operand
     publish();
   }
-  if (slot >= 0) {
+  if (MODE == SEG_STATE) {
+    float* e = entry(seg);
+    each([&](float& x, int r, int c) { e[r * CP + c] = x; });
+    each_n([&](float& a, float& b, int r) { if ((lane & 3) == 0) e[SegEntry<NT>::N + r] = a + b; });
+  } else if (slot >= 0 && seg == last_seg) {
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
@@ -804,26 +890,49 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
             const int r = srow + i * 16 + 8 * y;
             if (r < p.N) vecs[r] = ns[i][2 * y] + ns[i][2 * y + 1];
           }
-      if (sw == 0 && lane == 0) vecs[p.N] = m * (1.f / LOG2E);
+      if (warp == PREP && lane == 0) vecs[p.N] = m * (1.f / LOG2E);
     }
   }
 }
 
-template <int NT, bool ML>
-int launch_chunk(const ScanParams& p, int nseq, cudaStream_t st) {
+// Segments per sequence: as many as give the SMs two CTAs each, of at least 8 chunks, where there is room for two or more.
+inline int scan_segments(int longest, int nseq, int heads, int P) {
+  const long long ctas = (long long)((P + CP - 1) / CP) * heads * nseq, room = 2LL * dlti_num_sms() / (ctas > 0 ? ctas : 1);
+  const int most = longest / (8 * CQ);
+  const int segs = (int)(room < most ? room : most);
+  return segs > 1 ? (segs < 16 ? segs : 16) : 1;
+}
+
+template <int NT, bool ML, int MODE>
+int launch_chunk_mode(const ScanParams& p, int nseq, int conv_parts, cudaStream_t st) {
   static bool done[64] = {};
   const int bytes = ML ? ChunkSmem<NT>::BYTES_ML : ChunkSmem<NT>::BYTES;
   int dev = 0;
   DLTI_CUDA_CHECK(cudaGetDevice(&dev));
   if (!done[dev & 63]) {
-    DLTI_CUDA_CHECK(cudaFuncSetAttribute(scan_chunk_kernel<NT, ML>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    DLTI_CUDA_CHECK(cudaFuncSetAttribute(scan_chunk_kernel<NT, ML, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     done[dev & 63] = true;
   }
   const int slices = (p.P + CP - 1) / CP;
-  const int conv_parts = p.conv_state ? (p.conv_C + 2047) / 2048 : 0;
-  scan_chunk_kernel<NT, ML><<<dim3(slices + conv_parts, p.heads, nseq), 256, bytes, st>>>(p, slices, conv_parts);
+  scan_chunk_kernel<NT, ML, MODE><<<dim3(slices + conv_parts, p.heads, nseq * (MODE == WHOLE ? 1 : p.segs)), 256, bytes, st>>>(p, slices, conv_parts);
   dlti_count_launch();
   return (int)cudaGetLastError();
+}
+template <int NT, bool ML>
+int launch_chunk(const ScanParams& p, int nseq, cudaStream_t st) {
+  const int conv_parts = p.conv_state ? (p.conv_C + 2047) / 2048 : 0;
+  if (p.segs <= 1) return launch_chunk_mode<NT, ML, WHOLE>(p, nseq, conv_parts, st);
+  if (int rc = launch_chunk_mode<NT, ML, SEG_STATE>(p, nseq, 0, st)) return rc;
+  return launch_chunk_mode<NT, ML, SEG_FULL>(p, nseq, conv_parts, st);
+}
+inline int segment_floats(int N) { return N <= 64 ? SegEntry<64>::FLOATS : (N <= 128 ? SegEntry<128>::FLOATS : SegEntry<256>::FLOATS); }
+// segments of at most `longest` rows a sequence in ws (null: none)
+inline void set_segments(ScanParams& p, int longest, int nseq, float* ws) {
+  const int segs = ws ? scan_segments(longest, nseq, p.heads, p.P) : 1;
+  if (segs <= 1 || (long long)nseq * segs > 65535) return;
+  p.seg_len = ((longest + segs - 1) / segs + CQ - 1) / CQ * CQ;
+  p.segs = (longest + p.seg_len - 1) / p.seg_len;
+  p.seg_ws = ws;
 }
 
 // x = silu(x) in place, rounded to T
@@ -867,11 +976,13 @@ DLTI_API int dlti_linear_scan(const void* q, long long q_ld, const void* k, long
 
 // The chunked tensor-core form of the same for prompt sequences: bf16, N and P multiples of 8, N <= 256, q / k / v rows
 // 16-byte aligned, no silu (see dlti_silu_rows).
-DLTI_API int dlti_linear_scan_chunked(const void* q, long long q_ld, const void* k, long long k_ld, const void* v, long long v_ld, int rep,
+// longest and ws: rows of the longest of these sequences, and dlti_scan_workspace floats for cutting it into segments (null: whole).
+DLTI_API int dlti_linear_scan_split(const void* q, long long q_ld, const void* k, long long k_ld, const void* v, long long v_ld, int rep,
                                       const float* decay, const void* dt, long long dt_ld, const float* dt_bias, const float* A_log,
                                       const float* D, float* state, const int* sslot, const int* ctx, const int* cu, int nd, int seq0,
                                       int nseq, int heads, int N, int P, void* out, long long o_ld, const void* conv_src,
-                                      long long conv_ld, int conv_col, int conv_rows, int conv_C, void* conv_state, cudaStream_t st) {
+                                      long long conv_ld, int conv_col, int conv_rows, int conv_C, void* conv_state, int longest, float* ws,
+                                    cudaStream_t st) {
   if (nseq <= 0) return 0;
   if (heads < 1 || rep < 1 || nseq > 65535 || (!decay && (!dt || !dt_bias || !A_log))) return DLTI_ERR_BAD_ARG;
   if (N % 8 || P % 8 || q_ld % 8 || k_ld % 8 || v_ld % 8 || o_ld % 2 ||
@@ -882,6 +993,7 @@ DLTI_API int dlti_linear_scan_chunked(const void* q, long long q_ld, const void*
   if (conv_rows <= 0) conv_state = nullptr;
   ScanParams p{q, k, v, q_ld, k_ld, v_ld, rep, 0, decay, dt, dt_ld, dt_bias, A_log, D, state, sslot, ctx, cu,
                nd, seq0, heads, N, P, out, o_ld, conv_src, conv_ld, conv_col, conv_rows, conv_C, conv_state};
+  set_segments(p, longest, nseq, ws);
   if (N <= 64) return launch_chunk<64, false>(p, nseq, st);
   if (N <= 128) return launch_chunk<128, false>(p, nseq, st);
   if (N <= 256) return launch_chunk<256, false>(p, nseq, st);
@@ -889,13 +1001,30 @@ DLTI_API int dlti_linear_scan_chunked(const void* q, long long q_ld, const void*
   return DLTI_ERR_TOO_LARGE;
 }
 
+DLTI_API int dlti_linear_scan_chunked(const void* q, long long q_ld, const void* k, long long k_ld, const void* v, long long v_ld, int rep,
+                                      const float* decay, const void* dt, long long dt_ld, const float* dt_bias, const float* A_log,
+                                      const float* D, float* state, const int* sslot, const int* ctx, const int* cu, int nd, int seq0,
+                                      int nseq, int heads, int N, int P, void* out, long long o_ld, const void* conv_src,
+                                      long long conv_ld, int conv_col, int conv_rows, int conv_C, void* conv_state, cudaStream_t st) {
+  return dlti_linear_scan_split(q, q_ld, k, k_ld, v, v_ld, rep, decay, dt, dt_ld, dt_bias, A_log, D, state, sslot, ctx, cu, nd, seq0, nseq, heads,
+                                N, P, out, o_ld, conv_src, conv_ld, conv_col, conv_rows, conv_C, conv_state, 0, nullptr, st);
+}
+
+// floats of workspace with which the chunked forms cut sequences of up to `longest` rows into segments (0: they would not)
+DLTI_API long long dlti_scan_workspace(int longest, int nseq, int heads, int N, int P) {
+  if (nseq < 1 || heads < 1 || P < 1 || N < 1 || N > 256) return 0;
+  const int segs = scan_segments(longest, nseq, heads, P);
+  return segs > 1 ? (long long)nseq * segs * heads * ((P + CP - 1) / CP) * segment_floats(N) : 0;
+}
+
 // mLSTM over the sequences [seq0, seq0 + nseq): q, k rows heads * N, v rows heads * P wide; gates / gate_b: see ScanParams; state
 // [slots, heads, N, P], vec [slots, heads, ceil(P / 32), N + 1]. chunked: the tensor-core form (bf16, N and P multiples of 8,
 // N <= 256, 16-byte aligned rows), else token by token (N <= 512).
-DLTI_API int dlti_mlstm_scan(const void* q, long long q_ld, const void* k, long long k_ld, const void* v, long long v_ld, const float* gates,
+// longest, ws: see dlti_linear_scan_split.
+DLTI_API int dlti_mlstm_scan_split(const void* q, long long q_ld, const void* k, long long k_ld, const void* v, long long v_ld, const float* gates,
                              long long g_ld, const float* gate_b, float cap, float q_scale, float* state, float* vec, const int* sslot,
                              const int* ctx, const int* cu, int nd, int seq0, int nseq, int heads, int N, int P, void* out, long long o_ld,
-                             int chunked, int dtype, cudaStream_t st) {
+                             int chunked, int dtype, int longest, float* ws, cudaStream_t st) {
   if (nseq <= 0) return 0;
   if (heads < 1 || N < 1 || P < 1 || nseq > 65535 || !gates || !gate_b || !(cap > 0.f)) return DLTI_ERR_BAD_ARG;
   ScanParams p{};
@@ -912,9 +1041,18 @@ DLTI_API int dlti_mlstm_scan(const void* q, long long q_ld, const void* k, long 
     dlti_set_error("mlstm_scan, chunked: bf16, 16-byte aligned rows, N and P multiples of 8, N <= 256");
     return DLTI_ERR_BAD_ARG;
   }
+  set_segments(p, longest, nseq, ws);
   if (N <= 64) return launch_chunk<64, true>(p, nseq, st);
   if (N <= 128) return launch_chunk<128, true>(p, nseq, st);
   return launch_chunk<256, true>(p, nseq, st);
+}
+
+DLTI_API int dlti_mlstm_scan(const void* q, long long q_ld, const void* k, long long k_ld, const void* v, long long v_ld, const float* gates,
+                             long long g_ld, const float* gate_b, float cap, float q_scale, float* state, float* vec, const int* sslot,
+                             const int* ctx, const int* cu, int nd, int seq0, int nseq, int heads, int N, int P, void* out, long long o_ld,
+                             int chunked, int dtype, cudaStream_t st) {
+  return dlti_mlstm_scan_split(q, q_ld, k, k_ld, v, v_ld, gates, g_ld, gate_b, cap, q_scale, state, vec, sslot, ctx, cu, nd, seq0, nseq, heads,
+                               N, P, out, o_ld, chunked, dtype, 0, nullptr, st);
 }
 
 DLTI_API int dlti_silu_rows(void* x, long long ld, long long rows, int n, int dtype, cudaStream_t st) {

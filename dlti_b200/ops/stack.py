@@ -634,14 +634,20 @@ def _scan_tokens(q, k, v, decay, state, rows, seq0, nseq, heads, groups, N, P, s
                  _lib.dtype_code(v.dtype), _lib.stream_ptr()), "linear_scan")
 
 
+def _scan_workspace(rows, nseq, heads, N, P, device):
+    """Room for the states between the segments that the chunked kernels cut long prompts into, or None where they would not."""
+    n = _lib.fn("dlti_scan_workspace", [_I, _I, _I, _I, _I], restype=_L)(rows.max_seqlen, nseq, heads, N, P)
+    return torch.empty(n, dtype=torch.float32, device=device) if n else None
+
+
 def _scan_chunked(q, k, v, decay, state, rows, seq0, nseq, heads, groups, N, P, conv, out):
-    f = _lib.fn("dlti_linear_scan_chunked", [_V, _L, _V, _L, _V, _L, _I, _V, _V, _L, _V, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I,
-                                             _V, _L, _V, _L, _I, _I, _I, _V, _V])
-    dt = decay.dt
+    f = _lib.fn("dlti_linear_scan_split", [_V, _L, _V, _L, _V, _L, _I, _V, _V, _L, _V, _V, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I,
+                                           _V, _L, _V, _L, _I, _I, _I, _V, _I, _V, _V])
+    dt, ws = decay.dt, _scan_workspace(rows, nseq, heads, N, P, q.device)
     _lib.check(f(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), heads // groups, _p(decay.const), _p(dt),
                  0 if dt is None else dt.stride(0), _p(decay.dt_bias), _p(decay.A_log), _p(decay.D), _p(state), _p(rows.state),
                  _p(rows.ctx), _p(rows.cu), rows.nd, seq0, nseq, heads, N, P, _p(out), out.stride(0), *_conv_args(conv),
-                 _lib.stream_ptr()), "linear_scan_chunked")
+                 rows.max_seqlen, _p(ws), _lib.stream_ptr()), "linear_scan_split")
 
 
 def mlstm_scan_ref(q, k, v, gates, gate_b, cap, state, vec, rows: Rows, heads, N, P):
@@ -683,12 +689,14 @@ def mlstm_scan(q, k, v, gates, gate_b, cap, state, vec, rows: Rows, heads, N, P)
     if not _lib.use_native(q):
         return mlstm_scan_ref(q, k, v, gates, gate_b, cap, state, vec, rows, heads, N, P)
     out = act(q.shape[0], heads * P, v.dtype, q.device)
-    f = _lib.fn("dlti_mlstm_scan", [_V, _L, _V, _L, _V, _L, _V, _L, _V, _F, _F, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _V, _L, _I, _I, _V])
+    f = _lib.fn("dlti_mlstm_scan_split", [_V, _L, _V, _L, _V, _L, _V, _L, _V, _F, _F, _V, _V, _V, _V, _V, _I, _I, _I, _I, _I, _I, _V, _L, _I, _I,
+                                          _I, _V, _V])
 
     def run(seq0, nseq, chunked):
+        ws = _scan_workspace(rows, nseq, heads, N, P, q.device) if chunked else None
         _lib.check(f(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(gates), gates.stride(0), _p(gate_b), float(cap), N ** -0.5,
                      _p(state), _p(vec), _p(rows.state), _p(rows.ctx), _p(rows.cu), rows.nd, seq0, nseq, heads, N, P, _p(out), out.stride(0),
-                     int(chunked), _lib.dtype_code(v.dtype), _lib.stream_ptr()), "mlstm_scan")
+                     int(chunked), _lib.dtype_code(v.dtype), rows.max_seqlen, _p(ws), _lib.stream_ptr()), "mlstm_scan_split")
 
     nd, nseq = rows.nd, rows.nseq
     if nseq > nd and q.dtype == torch.bfloat16 and N % 8 == 0 and P % 8 == 0 and N <= 256 and rows.max_seqlen >= _CHUNKED_FROM:

@@ -414,6 +414,13 @@ int dlti_linear_scan_chunked(const void* q, long long q_ld, const void* k, long 
     float* D, float* state, const int* sslot, const int* ctx, const int* cu, int nd, int seq0, int nseq, int heads, int
     N, int P, void* out, long long o_ld, const void* conv_src, long long conv_ld, int conv_col, int conv_rows, int
     conv_C, void* conv_state, dlti_stream_t stream);
+/* the same; sequences of up to `longest` rows may be cut into segments that run side by side. ws: dlti_scan_workspace floats, or null */
+int dlti_linear_scan_split(const void* q, long long q_ld, const void* k, long long k_ld, const void* v, long long
+    v_ld, int rep, const float* decay, const void* dt, long long dt_ld, const float* dt_bias, const float* A_log, const
+    float* D, float* state, const int* sslot, const int* ctx, const int* cu, int nd, int seq0, int nseq, int heads, int
+    N, int P, void* out, long long o_ld, const void* conv_src, long long conv_ld, int conv_col, int conv_rows, int
+    conv_C, void* conv_state, int longest, float* ws, dlti_stream_t stream);
+long long dlti_scan_workspace(int longest, int nseq, int heads, int N, int P);
 /* x = silu(x) in place */
 int dlti_silu_rows(void* x, long long ld, long long rows, int n, int dtype, dlti_stream_t stream);
 /* paged attention, one warp per (row, head), fp32 arithmetic; chunk > 0: a position sees its own chunk only; window > 0: itself and the
@@ -445,6 +452,10 @@ int dlti_attn_fwd_split(const void* qkv, void* out, long long ldo, const float* 
 int dlti_mlstm_scan(const void* q, long long q_ld, const void* k, long long k_ld, const void* v, long long v_ld, const float* gates,
     long long g_ld, const float* gate_b, float cap, float q_scale, float* state, float* vec, const int* sslot, const int* ctx, const
     int* cu, int nd, int seq0, int nseq, int heads, int N, int P, void* out, long long o_ld, int chunked, int dtype, dlti_stream_t stream);
+/* longest, ws: as for dlti_linear_scan_split */
+int dlti_mlstm_scan_split(const void* q, long long q_ld, const void* k, long long k_ld, const void* v, long long v_ld, const float* gates,
+    long long g_ld, const float* gate_b, float cap, float q_scale, float* state, float* vec, const int* sslot, const int* ctx, const
+    int* cu, int nd, int seq0, int nseq, int heads, int N, int P, void* out, long long o_ld, int chunked, int dtype, int longest, float* ws, dlti_stream_t stream);
 /* streams.cu. Hyper-connections between two sublayers: x_t <- sum_s mix[s,t] x_s + out[t] y on x [rows, S, d] (y may be NULL), then
  * h = layer_norm(sum_s in[s] x_s) * w (w may be NULL), then (cw, one token per sequence) plus its causal convolution */
 int dlti_hyper(float* x, int S, int d, const void* y, long long y_ld, const float* mix, const float* out, const float* in, const float*

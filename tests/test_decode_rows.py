@@ -64,3 +64,39 @@ def test_fed_ids(n):
     ids, sampled = torch.randint(0, 1 << 40, (n,), generator=g), torch.randint(0, 1 << 40, (300,), generator=g)
     src = torch.randint(-1, 300, (n,), generator=g, dtype=torch.int32)
     assert torch.equal(S.feed_ids(ids.cuda(), src.cuda(), sampled.cuda()).cpu(), S.feed_ids(ids, src, sampled))
+
+
+@pytest.mark.parametrize("kind", ["mamba2", "lightning", "mlstm"])
+@pytest.mark.parametrize("lens,carried", [((1024,), 0), ((1025,), 7), ((1600, 30, 700), 5), ((512, 1537), 0)])
+@pytest.mark.parametrize("N,P", [(64, 32), (128, 40), (200, 24)])
+def test_prompts_in_segments(kind, N, P, lens, carried, monkeypatch):
+    """Segments of a prompt side by side give what the chain of all chunks gives; both have the same products, in another order."""
+    heads, T, dev = 2, 2 + sum(lens), "cuda"
+    g = torch.Generator().manual_seed(N + T)
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    q, k, v = (_act(x, dev, BF16) for x in (rnd(T, heads * N), rnd(T, heads * N) * 0.2, rnd(T, heads * P)))
+    z = rnd(T, 2 * heads)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    n = 2 + len(lens)
+    cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    rows = K.Rows(i32([0] * T), i32([0] * T), i32([0] * T).long(), i32([9, 1] + [x + carried for x in lens]), i32(cu), i32([[0]] * n),
+                  i32(list(range(n, 0, -1))), 2, max(lens), 4096)
+    assert K._scan_workspace(rows, len(lens), heads, N, P, dev) is not None
+    state, vec = rnd(n + 1, heads, N, P).to(dev), rnd(n + 1, heads, 1, N + 1).repeat(1, 1, -(-P // 32), 1).flatten(2).to(dev)
+    bias, A_log = torch.linspace(-4, 0, heads, device=dev), torch.linspace(-1, 1, heads, device=dev)
+    out = []
+    for split in (True, False):
+        if not split:
+            monkeypatch.setattr(K, "_scan_workspace", lambda *a: None)
+        st, vc = state.clone(), vec.clone()
+        if kind == "mlstm":
+            y = K.mlstm_scan(q, k, v, _act(z, dev, F32), torch.cat([bias, 4 - bias]), 15.0, st, vc, rows, heads, N, P)
+        elif kind == "lightning":
+            y = K.linear_scan(q, k, v, K.Decay(const=torch.tensor([0.999, 0.9], device=dev)), st, rows, heads, heads, N, P)
+        else:
+            dec = K.Decay(dt=_act(z[:, :heads], dev, BF16), dt_bias=bias, A_log=A_log, D=bias)
+            y = K.linear_scan(q, k, v, dec, st, rows, heads, heads, N, P)
+        out.append((y.double(), st.double(), vc.double()))
+    for a, b, tol in zip(*out, (2e-3, 2e-5, 2e-5)):              # outputs rounded to 8 bits; states: 16 bits and more in every product
+        assert bool(torch.isfinite(a).all()) and (a - b).norm() <= tol * b.norm()
+    assert torch.equal(out[0][1][0], state[0].double())
