@@ -32,8 +32,6 @@ from .kv_cache import KVCache, KVSpec
 _FUSE_ACC = os.environ.get("DLTI_DECODE_FUSE_ACC", "1") == "1"    # A/B switch: consume the fp32 accumulators directly
 
 
-# opt-in until measured on the serving shapes: prefill gate_up GEMM with SwiGLU in its epilogue (the training kernel)
-_PREFILL_FUSE_SWIGLU = os.environ.get("DLTI_SERVE_FUSE_SWIGLU", "0") == "1"
 _TP_LARGE = os.environ.get("DLTI_TP_LARGE_RSAG", "1") == "1"          # prefill-sized steps: reduce-scatter + all-gather
 # how prefill-sized steps do it: "fused" = reduce-scatter in the row-parallel GEMM's epilogue (K10) and all-gather in
 # the next column-parallel GEMM's producer (K11); "pull" = the round-1 stand-alone pull-reduce-push kernel
@@ -450,8 +448,9 @@ class ModelRunner:
                 xn = row_reduce(attn, lw["w_o"], lw["ln2"])
             if acc_path:
                 h = E.acc_swiglu(gemm_skinny_acc(xn, lw["w_gu"]), xn.dtype)
-            elif _PREFILL_FUSE_SWIGLU and not skinny:
-                # SwiGLU in the CTA-pair GEMM epilogue (falls back by itself)
+            elif not skinny:
+                # SwiGLU in the CTA-pair GEMM's epilogue (falls back by itself): 4 layers of 7B over 7400 prompt rows spent 517 us
+                # in the kernel of its own, now 58 more in the GEMMs
                 h = (gemm_swiglu(xn.rows(), lw["w_gu"], gather=xn.handle) if isinstance(xn, ShardedAct)
                      else gemm_swiglu(xn, lw["w_gu"]))
             else:
