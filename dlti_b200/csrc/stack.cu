@@ -22,6 +22,30 @@ __global__ void embed_rows_kernel(const long long* __restrict__ ids, const T* __
   }
 }
 
+// The same, a token per CTA in pieces of 8 (bf16, d a multiple of 8, aligned rows): 8192 tokens of 2048 (134 MB moved) in 23 instead of
+// 68 us. Every element cost the kernel above a 64-bit division and 2-byte accesses.
+__global__ void __launch_bounds__(256) embed_rows_vec_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
+                                                             float* __restrict__ x, __nv_bfloat16* __restrict__ xa, long long xa_ld, int d,
+                                                             long long vocab) {
+  griddep_pass();
+  const long long t = blockIdx.x, id = ids[t];
+  const bool ok = id >= 0 && id < vocab;
+  for (int c = threadIdx.x * 8; c < d; c += blockDim.x * 8) {
+    const int4 v = ok ? *reinterpret_cast<const int4*>(table + id * d + c) : make_int4(0, 0, 0, 0);
+    const uint32_t* u = reinterpret_cast<const uint32_t*>(&v);
+    float f[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 p = Cvt<__nv_bfloat16>::unpack2(u[j]);
+      f[2 * j] = p.x;
+      f[2 * j + 1] = p.y;
+    }
+    st8(x + t * d + c, f);
+    if (xa) *reinterpret_cast<int4*>(xa + t * xa_ld + c) = v;
+  }
+}
+inline unsigned piece_threads(int d) { return (unsigned)(d / 8 >= 256 ? 256 : (d / 8 + 31) / 32 * 32); }
+
 // out = scale * acc (fp32), with cap > 0: cap * tanh(scale * acc / cap); clear: acc = 0 (otherwise out may be acc)
 __global__ void take_rows_kernel(float* acc, float* out, float scale, float cap, int clear, long long vec) {
   griddep_pass();
@@ -966,6 +990,13 @@ int gated_norm_mode(const void* y, long long y_ld, const void* gate, long long g
 DLTI_API int dlti_embed_rows(const long long* ids, const void* table, float* x, void* xa, long long xa_ld, long long tokens,
                              int d, long long vocab, int dtype, cudaStream_t st) {
   if (tokens <= 0) return 0;
+  const uintptr_t al = reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(xa);
+  if (dtype == DLTI_BF16 && d % 8 == 0 && (!xa || xa_ld % 8 == 0) && (al & 15) == 0 && tokens <= 0x7fffffff) {
+    DLTI_CUDA_CHECK(dlti_launch_pdl(tokens, embed_rows_vec_kernel, dim3((unsigned)tokens), dim3(piece_threads(d)), 0, st, ids,
+                                    (const __nv_bfloat16*)table, x, (__nv_bfloat16*)xa, xa_ld, d, vocab));
+    dlti_count_launch();
+    return 0;
+  }
   const int g = grid_for(tokens * d, 256);
   DISPATCH_T(dtype, DLTI_CUDA_CHECK(dlti_launch_pdl(tokens, embed_rows_kernel<T>, dim3(g), dim3(256), 0, st, ids, (const T*)table, x,
                                                     (T*)xa, xa_ld, tokens, d, vocab)));

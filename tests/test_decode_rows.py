@@ -100,3 +100,22 @@ def test_prompts_in_segments(kind, N, P, lens, carried, monkeypatch):
     for a, b, tol in zip(*out, (2e-3, 2e-5, 2e-5)):              # outputs rounded to 8 bits; states: 16 bits and more in every product
         assert bool(torch.isfinite(a).all()) and (a - b).norm() <= tol * b.norm()
     assert torch.equal(out[0][1][0], state[0].double())
+
+
+@pytest.mark.parametrize("n,d", [(1, 8), (5, 40), (300, 2048), (7, 4104)])
+def test_embedded_rows_by_pieces(n, d):
+    from dlti_b200.ops import streams as H
+    g = torch.Generator().manual_seed(d)
+    table, ids = torch.randn(50, d, generator=g).to(BF16), torch.randint(0, 50, (n,), generator=g)
+    x, h = K.embed_rows(ids.cuda(), table.cuda())
+    assert torch.equal(x.cpu(), table[ids].float()) and torch.equal(h.cpu(), table[ids])
+    assert torch.equal(H.embed_streams(ids.cuda(), table.cuda(), 3, 2.5).cpu(), (table[ids].float() * 2.5)[:, None].expand(n, 3, d))
+
+
+@pytest.mark.parametrize("n,w", [(1, 8), (5, 2048), (6, 2056), (131, 6144)])
+def test_silu_of_rows(n, w):
+    x = torch.randn(n, w + 16, generator=torch.Generator().manual_seed(w)).to(BF16).cuda()
+    want = x.clone()
+    want[:, :w] = torch.nn.functional.silu(x[:, :w].float()).to(BF16)
+    K.silu_rows_(x[:, :w])
+    assert torch.equal(x[:, w:], want[:, w:]) and (x.float() - want.float()).abs().max() <= 2 ** -8 * want.float().abs().max()
