@@ -4,14 +4,18 @@
 //
 //   attn_prefill_kernel  portions of prompts, bf16: a CTA owns 128 (token, head of a group) rows and streams key / value
 //                        tiles of 64 from the pages through shared memory into mma.sync
-//   attn_decode_kernel   one new token per sequence, bf16: the query heads of a group share every key and value (rows of
-//                        one m16 fragment), keys are split over CTAs and the splits combined by attn_combine_kernel
+//   attn_decode_kernel   one new token per sequence, bf16 or fp16: the query heads of a group share every key and value (rows of
+//                        one m16 fragment), keys are split over CTAs: up to 8 of them are a cluster and exchange their
+//                        results through shared memory, more leave them to attn_combine_kernel
 //   attn_rows_kernel     one warp per (row, head), fp32 arithmetic throughout: the fp32 mode, and heads above 256
 //
-// Scores, softmax weights and sums are fp32. The weights enter the P*V product as two bf16 terms (hi + lo, 16 mantissa
-// bits), so the product is that of the fp32 weights with the bf16 values.
+// Scores, softmax weights and sums are fp32. The weights enter the P*V product as two 16-bit terms (hi + lo, 16 mantissa
+// bits and more), so the product is that of the fp32 weights with the 16-bit values.
 #include "mma_sync.cuh"
+#include "pair.cuh"
 #include "rows.cuh"
+
+#include <type_traits>
 
 namespace {
 
@@ -186,14 +190,14 @@ __device__ __forceinline__ void tile_slots(int* slots, const PagedParams& p, con
   }
 }
 // this thread's elements of query rows as A fragments; q0 / q1: rows lane / 4 and lane / 4 + 8 (null: zeros)
-template <int DK>
-__device__ __forceinline__ void load_q(uint32_t (&qf)[DK / 16][4], const bf16* q0, const bf16* q1, int dim) {
+template <int DK, typename T>
+__device__ __forceinline__ void load_q(uint32_t (&qf)[DK / 16][4], const T* q0, const T* q1, int dim) {
   const int c0 = (threadIdx.x & 3) * 2;
 #pragma unroll
   for (int kk = 0; kk < DK / 16; ++kk)
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
-      const bf16* q = (x & 1) ? q1 : q0;
+      const T* q = (x & 1) ? q1 : q0;
       const int c = kk * 16 + c0 + (x >> 1) * 8;
       uint32_t v = 0;
       if (q && c + 1 < dim) v = *reinterpret_cast<const uint32_t*>(q + c);
@@ -202,7 +206,7 @@ __device__ __forceinline__ void load_q(uint32_t (&qf)[DK / 16][4], const bf16* q
     }
 }
 // S[16 x 16 keys] of keys kt .. kt + 15 of the tile
-template <int DK>
+template <int DK, typename T = bf16>
 __device__ __forceinline__ void scores16(float (&s0)[4], float (&s1)[4], const uint32_t (&qf)[DK / 16][4], uint32_t k_base, int kt) {
   const int lane = threadIdx.x & 31;
   const uint32_t addr = k_base + ((kt + (lane & 7) + ((lane >> 4) << 3)) * (DK + 8) + ((lane >> 3) & 1) * 8) * 2;
@@ -210,28 +214,28 @@ __device__ __forceinline__ void scores16(float (&s0)[4], float (&s1)[4], const u
   for (int kk = 0; kk < DK / 16; ++kk) {
     uint32_t b[4];
     ldsm4(b, addr + kk * 32);
-    mma_bf16(s0, qf[kk], b[0], b[1]);
-    mma_bf16(s1, qf[kk], b[2], b[3]);
+    mma_16<T>(s0, qf[kk], b[0], b[1]);
+    mma_16<T>(s1, qf[kk], b[2], b[3]);
   }
 }
 // O += P[16 x 16 keys] V, the weights as hi + lo
-template <int DV>
+template <int DV, typename T = bf16>
 __device__ __forceinline__ void weighted16(float (&o)[DV / 8][4], const float (&p0)[4], const float (&p1)[4], uint32_t v_base, int kt) {
   const int lane = threadIdx.x & 31;
   uint32_t hi[4], lo[4];
-  split_pair(p0[0], p0[1], hi[0], lo[0]);
-  split_pair(p0[2], p0[3], hi[1], lo[1]);
-  split_pair(p1[0], p1[1], hi[2], lo[2]);
-  split_pair(p1[2], p1[3], hi[3], lo[3]);
+  split_pair_16<T>(p0[0], p0[1], hi[0], lo[0]);
+  split_pair_16<T>(p0[2], p0[3], hi[1], lo[1]);
+  split_pair_16<T>(p1[0], p1[1], hi[2], lo[2]);
+  split_pair_16<T>(p1[2], p1[3], hi[3], lo[3]);
   const uint32_t addr = v_base + ((kt + (lane & 15)) * (DV + 8) + (lane >> 4) * 8) * 2;
 #pragma unroll
   for (int d = 0; d < DV / 16; ++d) {
     uint32_t b[4];
     ldsm4_t(b, addr + d * 32);
-    mma_bf16(o[2 * d], hi, b[0], b[1]);
-    mma_bf16(o[2 * d], lo, b[0], b[1]);
-    mma_bf16(o[2 * d + 1], hi, b[2], b[3]);
-    mma_bf16(o[2 * d + 1], lo, b[2], b[3]);
+    mma_16<T>(o[2 * d], hi, b[0], b[1]);
+    mma_16<T>(o[2 * d], lo, b[0], b[1]);
+    mma_16<T>(o[2 * d + 1], hi, b[2], b[3]);
+    mma_16<T>(o[2 * d + 1], lo, b[2], b[3]);
   }
 }
 
@@ -385,11 +389,22 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const PagedParams p) 
   }
 }
 
-// grid (splits, G * head blocks of 16, sequences), 4 warps; warp w takes keys 16 w .. 16 w + 15 of every tile.
-template <int DK, int DV>
+// shared memory of another CTA of the cluster
+__device__ __forceinline__ float ld_peer_f32(uint32_t addr, uint32_t rank) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(mapa_rank(addr, rank)) : "memory");
+  return v;
+}
+
+// grid (splits, G * head blocks of 16, sequences), 4 warps; warp w takes keys 16 w .. 16 w + 15 of every tile. A short context is a
+// chain of latencies (context length, page table, keys, products, merge), so what counts is the number of steps and launches:
+// CLUSTER: the splits of a head are one cluster, whose CTAs merge each a part of the columns, in the place of a second kernel.
+// fp16 weights are scaled by 2^8 against their subnormals; it cancels in the division.
+template <typename T, int DK, int DV, bool CLUSTER>
 __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, int splits, float* __restrict__ part_o,
                                                          float* __restrict__ part_ml) {
   using L = Tile<DK, DV>;
+  constexpr float LIFT = std::is_same<T, __half>::value ? 8.f : 0.f;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ int s_slots[2][KT];
   __shared__ float s_m[4][16], s_l[4][16];
@@ -416,9 +431,9 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, i
     __syncthreads();
     load_tile<DK, DV>(sbase, p, walk, s_slots[0], g, jbeg, jend);
     uint32_t qf[DK / 16][4];
-    const bf16* q = reinterpret_cast<const bf16*>(p.q) + (long long)b * p.q_ld + (long long)(g * rep + h0) * p.q_hd;
+    const T* q = reinterpret_cast<const T*>(p.q) + (long long)b * p.q_ld + (long long)(g * rep + h0) * p.q_hd;
     const int r0 = lane >> 2, r1 = r0 + 8;
-    load_q<DK>(qf, r0 < nh ? q + (long long)r0 * p.q_hd : nullptr, r1 < nh ? q + (long long)r1 * p.q_hd : nullptr, p.dim);
+    load_q<DK, T>(qf, r0 < nh ? q + (long long)r0 * p.q_hd : nullptr, r1 < nh ? q + (long long)r1 * p.q_hd : nullptr, p.dim);
     const float sl2 = p.scale * LOG2E_F;
     int it = 0;
     for (int j0 = jbeg; j0 < jend; j0 += KT, ++it) {
@@ -436,7 +451,7 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, i
       const uint32_t kb = sbase + (it & 1) * L::BYTES, vb = kb + L::K_BYTES;
       float s[2][4] = {};
       const bool near = p.bias && ctx - (j0 + KT) < p.span;
-      scores16<DK>(s[0], s[1], qf, kb, warp * 16);
+      scores16<DK, T>(s[0], s[1], qf, kb, warp * 16);
       float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
       for (int i = 0; i < 2; ++i)
@@ -465,10 +480,10 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, i
       for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
-          s[i][x] = ex2(s[i][x] - m[x >> 1]);
+          s[i][x] = ex2(s[i][x] - m[x >> 1] + LIFT);
           l[x >> 1] += s[i][x];
         }
-      weighted16<DV>(o, s[0], s[1], vb, warp * 16);
+      weighted16<DV, T>(o, s[0], s[1], vb, warp * 16);
     }
   }
   // merge the four warps; the stages are free after the barrier
@@ -489,6 +504,20 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, i
     for (int x = 0; x < 4; ++x)
       so[(warp * 16 + (lane >> 2) + 8 * (x >> 1)) * DV + i * 8 + (lane & 3) * 2 + (x & 1)] = o[i][x];
   __syncthreads();
+  float* own = so + 4 * 16 * DV;                   // CLUSTER: this CTA's merged [16][vdim]; its maxima and sums go to s_m[0], s_l[0]
+  float row_m = 0.f, row_l = 0.f;
+  if (CLUSTER && threadIdx.x < 16) {
+    row_m = fmaxf(fmaxf(s_m[0][threadIdx.x], s_m[1][threadIdx.x]), fmaxf(s_m[2][threadIdx.x], s_m[3][threadIdx.x]));
+#pragma unroll
+    for (int w = 0; w < 4; ++w) row_l += s_m[w][threadIdx.x] == -INFINITY ? 0.f : s_l[w][threadIdx.x] * ex2(s_m[w][threadIdx.x] - row_m);
+  }
+  auto write = [&](int r, int c, float gm, float gl, float a) {
+    const int h = g * rep + h0 + r;
+    gl = with_sink(p, h, gm, gl);
+    float f = gl > 0.f ? 1.f / gl : 0.f;
+    if (p.gate) f *= p.gate[(long long)b * p.H + h];
+    reinterpret_cast<T*>(p.out)[(long long)b * p.o_ld + (long long)h * p.vdim + c] = Cvt<T>::from_f(a * f * gate_at<T>(p, b, h, c));
+  };
   for (int i = threadIdx.x; i < nh * p.vdim; i += 128) {
     const int r = i / p.vdim, c = i - r * p.vdim;
     float gm = -INFINITY, a = 0.f, gl = 0.f;
@@ -500,14 +529,12 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, i
       a += so[(w * 16 + r) * DV + c] * f;
       gl += s_l[w][r] * f;
     }
-    const int h = g * rep + h0 + r;
-    if (splits == 1) {
-      gl = with_sink(p, h, gm, gl);
-      float f = gl > 0.f ? 1.f / gl : 0.f;
-      if (p.gate) f *= p.gate[(long long)b * p.H + h];
-      reinterpret_cast<bf16*>(p.out)[(long long)b * p.o_ld + (long long)h * p.vdim + c] = __float2bfloat16(a * f * gate_at<bf16>(p, b, h, c));
+    if (CLUSTER) {
+      own[i] = a;
+    } else if (splits == 1) {
+      write(r, c, gm, gl, a);
     } else {
-      const long long idx = ((long long)b * p.H + h) * splits + split;
+      const long long idx = ((long long)b * p.H + g * rep + h0 + r) * splits + split;
       part_o[idx * p.vdim + c] = a;
       if (c == 0) {
         part_ml[idx * 2] = gm;
@@ -515,8 +542,38 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, i
       }
     }
   }
+  if constexpr (CLUSTER) {
+    __syncthreads();                               // s_m and s_l have been read
+    if (threadIdx.x < 16) {
+      s_m[0][threadIdx.x] = row_m;
+      s_l[0][threadIdx.x] = row_l;
+    }
+    __syncwarp();
+    cluster_sync_all();
+    const uint32_t am = smem_u32(&s_m[0][0]), al = smem_u32(&s_l[0][0]), ao = smem_u32(own);
+    for (int i = split * 128 + threadIdx.x; i < nh * p.vdim; i += splits * 128) {
+      const int r = i / p.vdim;
+      float ms[8], gm = -INFINITY, a = 0.f, gl = 0.f;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        ms[s] = s < splits ? ld_peer_f32(am + r * 4, s) : -INFINITY;
+        gm = fmaxf(gm, ms[s]);
+      }
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (ms[s] != -INFINITY) {
+          const float f = ex2(ms[s] - gm);
+          a += ld_peer_f32(ao + i * 4, s) * f;
+          gl += ld_peer_f32(al + r * 4, s) * f;
+        }
+      write(r, i - r * p.vdim, gm, gl, a);
+    }
+    __syncwarp();                                  // nobody leaves while its shared memory is read; nothing has to be released
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+  }
 }
 
+template <typename T>
 __global__ void __launch_bounds__(128) attn_combine_kernel(const PagedParams p, int splits, const float* __restrict__ part_o,
                                                           const float* __restrict__ part_ml) {
   griddep_pass();
@@ -537,7 +594,7 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(const PagedParams p, 
       const float ms = part_ml[(base + s) * 2];
       if (ms != -INFINITY) a += part_o[(base + s) * p.vdim + c] * ex2(ms - gm);
     }
-    reinterpret_cast<bf16*>(p.out)[(long long)b * p.o_ld + (long long)h * p.vdim + c] = __float2bfloat16(a * f * gate_at<bf16>(p, b, h, c));
+    reinterpret_cast<T*>(p.out)[(long long)b * p.o_ld + (long long)h * p.vdim + c] = Cvt<T>::from_f(a * f * gate_at<T>(p, b, h, c));
   }
 }
 
@@ -565,23 +622,27 @@ int launch_prefill(const PagedParams& p, int nseq, int max_rows, cudaStream_t st
   return (int)cudaGetLastError();
 }
 
-template <int DK, int DV>
-int launch_decode(const PagedParams& p, int splits, float* ws, cudaStream_t st) {
-  static bool done[64] = {};
-  const int merge = 4 * 16 * DV * 4, smem = 2 * Tile<DK, DV>::BYTES > merge ? 2 * Tile<DK, DV>::BYTES : merge;
-  if (int rc = allow_smem(attn_decode_kernel<DK, DV>, smem, done)) return rc;
+template <typename T, int DK, int DV>
+int launch_decode_t(const PagedParams& p, int splits, float* ws, cudaStream_t st) {
+  static bool done[2][64] = {};
+  constexpr int merge = 5 * 16 * DV * 4, tiles = 2 * Tile<DK, DV>::BYTES, smem = tiles > merge ? tiles : merge;
+  const bool cluster = splits > 1 && splits <= 8;
+  auto kern = cluster ? attn_decode_kernel<T, DK, DV, true> : attn_decode_kernel<T, DK, DV, false>;
+  if (int rc = allow_smem(kern, smem, done[cluster])) return rc;
   const int rep = p.H / p.G;
-  float* part_ml = ws + (long long)p.rows * p.H * splits * p.vdim;
-  DLTI_CUDA_CHECK(dlti_launch_pdl(p.rows, attn_decode_kernel<DK, DV>, dim3(splits, p.G * ((rep + 15) / 16), (unsigned)p.rows), dim3(128),
-                                  (size_t)smem, st, p, splits, ws, part_ml));
+  float* part_ml = cluster ? nullptr : ws + (long long)p.rows * p.H * splits * p.vdim;
+  DLTI_CUDA_CHECK(dlti_launch_pdl_cluster(p.rows, cluster ? splits : 1, kern, dim3(splits, p.G * ((rep + 15) / 16), (unsigned)p.rows), dim3(128),
+                                          (size_t)smem, st, p, splits, ws, part_ml));
   dlti_count_launch();
-  if (splits > 1) {
-    DLTI_CUDA_CHECK(dlti_launch_pdl(p.rows, attn_combine_kernel, dim3(p.H, (unsigned)p.rows), dim3(128), 0, st, p, splits,
+  if (splits > 1 && !cluster) {
+    DLTI_CUDA_CHECK(dlti_launch_pdl(p.rows, attn_combine_kernel<T>, dim3(p.H, (unsigned)p.rows), dim3(128), 0, st, p, splits,
                                     (const float*)ws, (const float*)part_ml));
     dlti_count_launch();
   }
   return 0;
 }
+template <int DK, int DV>
+int launch_decode(const PagedParams& p, int splits, float* ws, cudaStream_t st) { return launch_decode_t<bf16, DK, DV>(p, splits, ws, st); }
 
 #define HEAD_DISPATCH(dim, vdim, F, ...)                                \
   do {                                                                  \
@@ -650,4 +711,15 @@ DLTI_API int dlti_attn_paged_decode(const void* q, long long q_ld, int q_hd, con
   PagedParams p{q, q_ld, q_hd, kc, vc, kd, vd, tables, max_blocks, bs, ctx, nullptr, nullptr, nullptr, 0, H, G, dim, vdim, chunk, window, scale, cap,
                 gate, out, o_ld, batch, sink, bias, span, ogate, og_ld};
   HEAD_DISPATCH(kd, vd, launch_decode, p, splits, ws, st);
+}
+
+// bf16 or fp16, heads of 128: decode attention of a model whose query heads share key / value heads (see dlti_paged_decode)
+int dlti_paged_decode_groups(const void* q, long long q_ld, const void* kc, const void* vc, const int* tables, int max_blocks, const int* ctx,
+                             int batch, int bs, int H, int G, float scale, int splits, float* ws, void* out, long long o_ld, int dtype,
+                             cudaStream_t st) {
+  PagedParams p{q, q_ld, 128, kc, vc, 128, 128, tables, max_blocks, bs, ctx, nullptr, nullptr, nullptr, 0, H, G, 128, 128, 0, 0, scale, 0.f,
+                nullptr, out, o_ld, batch, nullptr, nullptr, 0, nullptr, 0};
+  if (dtype == DLTI_BF16) return launch_decode_t<bf16, 128, 128>(p, splits, ws, st);
+  if (dtype == DLTI_FP16) return launch_decode_t<__half, 128, 128>(p, splits, ws, st);
+  return DLTI_ERR_UNSUPPORTED;
 }

@@ -70,20 +70,33 @@ int dlti_get_tmap_mn3d(CUtensorMap* out, const void* base, uint64_t N, uint64_t 
 // and 655 instead of 727 us on 6 Logozen layers; at 64 rows of 4 Llama-2-7B layers, where the weights take most of it, 678 and
 // 680 us. Larger steps fall back to plain stream ordering: their kernels fill the GPU.
 constexpr long long DLTI_PDL_MAX_ROWS = 256;
+// cluster > 1: CTAs of a cluster along x.
 template <typename... KArgs, typename... Args>
-inline cudaError_t dlti_launch_pdl(long long rows, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                   cudaStream_t stream, Args... args) {
+inline cudaError_t dlti_launch_pdl_cluster(long long rows, int cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                           cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
-  cfg.numAttrs = (dlti_pdl_enabled() && rows <= DLTI_PDL_MAX_ROWS) ? 1 : 0;
+  if (dlti_pdl_enabled() && rows <= DLTI_PDL_MAX_ROWS) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t dlti_launch_pdl(long long rows, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                   Args... args) {
+  return dlti_launch_pdl_cluster(rows, 1, kernel, grid, block, smem, stream, args...);
 }
 
 // ---------------------------------------------------------------------------

@@ -82,6 +82,13 @@ _ws: dict = {}
 _ws_retired: list = []
 
 
+def decode_splits(ctas: int, reach: int) -> int:
+    """CTAs over which the grouped decode attention cuts contexts of up to `reach` keys (tiles of 64) when one each would be `ctas`: one
+    wave of three per SM. Up to 8 are a cluster and merge by themselves; more are combined by a second kernel (8 CTAs with two tiles
+    each in their place took as long: 4 sequences of 1000 keys)."""
+    return max(1, min(32, 3 * 148 // max(1, ctas), -(-reach // 64)))
+
+
 def paged_decode(q, k_cache, v_cache, block_tables, ctx_lens, H, KV, hd, scale=None, out=None,
                  max_ctx: int | None = None):
     """q: [B, >= H*hd] (row b = the single new token of sequence b; head h at columns h*hd..).
@@ -101,8 +108,8 @@ def paged_decode(q, k_cache, v_cache, block_tables, ctx_lens, H, KV, hd, scale=N
     mc = max_ctx if max_ctx is not None else block_tables.shape[1] * bs
     # enough CTAs (128 threads each, ~4 resident per SM) to fill the machine: short contexts are latency-bound,
     # so small batches are cut into more KV splits
-    sms = 148
-    splits = max(1, min(16, -(-(4 * sms) // max(1, B * H)), (mc + 255) // 256))
+    grouped = H > KV and B * H >= 64              # the kernel that dlti_paged_decode takes
+    splits = decode_splits(B * KV * -(-(H // KV) // 16), mc) if grouped else max(1, min(16, -(-(4 * 148) // max(1, B * H)), (mc + 255) // 256))
     need = _lib.fn("dlti_paged_decode_workspace_floats", [_I, _I, _I], C.c_int)(B, H, splits)
     key = str(q.device)
     ws = _ws.get(key)

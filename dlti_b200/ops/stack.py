@@ -13,6 +13,7 @@ import torch
 from ..models.stack import round8
 from . import _debug, _lib
 from .gemm import gemm, gemm_skinny, gemm_skinny_acc
+from .serving import decode_splits
 
 _V, _I, _L, _F = C.c_void_p, C.c_int, C.c_longlong, C.c_float
 _p = _lib.ptr
@@ -443,8 +444,8 @@ def attn_paged_decode(q, m, rows: Rows, kc, vc, gate, out, splits: int | None = 
     if splits is None:
         reach = min(rows.max_ctx or 1 << 30, m.chunk or m.window or 1 << 30, rows.tables.shape[1] * bs)
         ctas = max(1, B) * m.kv_heads * -(-(m.heads // m.kv_heads) // 16)
-        splits = max(1, min(32, 3 * 148 // ctas, -(-reach // 64)))     # one wave of three CTAs per SM
-    ws = _workspace(q.device, B * m.heads * splits * (m.vdim + 2)) if splits > 1 else None
+        splits = decode_splits(ctas, reach)
+    ws = _workspace(q.device, B * m.heads * splits * (m.vdim + 2)) if splits > 8 else None
     f = _lib.fn("dlti_attn_paged_decode", [_V, _L, _I, _V, _V, _I, _I, _V, _I, _I, _V, _I, _I, _I, _I, _I, _I, _I, _F, _F, _V, _V, *_MORE, _I, _V, _V, _L, _V])
     _lib.check(f(_p(q), q.stride(0), hd, _p(kc), _p(vc), kc.shape[3], vc.shape[3], _p(rows.tables), rows.tables.shape[1], bs,
                  _p(rows.ctx), B, m.heads, m.kv_heads, m.dim, m.vdim, m.chunk, m.window, m.scale, m.softcap, _p(gate), _p(sink),

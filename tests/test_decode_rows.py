@@ -102,6 +102,26 @@ def test_prompts_in_segments(kind, N, P, lens, carried, monkeypatch):
     assert torch.equal(out[0][1][0], state[0].double())
 
 
+@pytest.mark.parametrize("dtype,tol", [(BF16, 4e-3), (torch.float16, 6e-4)])       # outputs rounded to 8 and 11 bits
+@pytest.mark.parametrize("max_ctx", [64, 400, 4096])                               # one CTA, a cluster, more than a cluster
+@pytest.mark.parametrize("H,KV,bs", [(4, 2, 16), (8, 2, 16), (16, 1, 24), (20, 1, 16), (51, 3, 16)])
+def test_decode_attention_of_shared_heads(H, KV, bs, max_ctx, dtype, tol):
+    from dlti_b200.ops import serving as S
+    g = torch.Generator().manual_seed(H)
+    ctx = [c for c in (1, 15, 63, 64, 65, 129, 400, 700, 4096) if c <= max_ctx]
+    ctx += [37] * (-(-64 // H) - len(ctx))                        # the rows from which the heads of a group go together
+    nb = [-(-c // bs) for c in ctx]
+    tables, kc, vc = torch.zeros(len(ctx), max(nb), dtype=torch.int32), *(torch.randn(sum(nb), bs, KV, 128, generator=g).to(dtype) for _ in range(2))
+    perm, at = torch.randperm(sum(nb), generator=g).int(), 0
+    for i, n in enumerate(nb):
+        tables[i, :n] = perm[at:at + n]
+        at += n
+    q, lens = torch.randn(len(ctx), H * 128, generator=g).to(dtype) * 2, torch.tensor(ctx, dtype=torch.int32)
+    want = S.paged_decode_ref(q.float(), kc.float(), vc.float(), tables, lens, H, KV, 128, 128 ** -0.5)
+    got = S.paged_decode(q.cuda(), kc.cuda(), vc.cuda(), tables.cuda(), lens.cuda(), H, KV, 128, max_ctx=max_ctx).cpu()
+    assert bool(((got.float() - want).norm(dim=1) <= tol * want.norm(dim=1)).all())
+
+
 @pytest.mark.parametrize("n,d", [(1, 8), (5, 40), (300, 2048), (7, 4104)])
 def test_embedded_rows_by_pieces(n, d):
     from dlti_b200.ops import streams as H
