@@ -91,7 +91,8 @@ def check(rc: int, what: str = "") -> None:
 
 
 def stream_ptr() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the handle itself: building a torch.cuda.Stream around it took longer than the rest of a launch's bookkeeping
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def ptr(t: torch.Tensor | None) -> C.c_void_p:
