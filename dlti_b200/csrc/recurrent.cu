@@ -385,33 +385,36 @@ int launch_scan(const ScanParams& p, int nseq, cudaStream_t st) {
 // n . q the row sums of the bracketed weights plus one more column of S^T q.
 //
 // One sequence gives only heads * P / 32 CTAs, each a chain of n / 64 chunks. Where that leaves SMs without work, the sequence is
-// cut into segments of whole chunks: a first launch (SEG_STATE) runs the state half alone over every segment but the last, from
-// zero (the first one from the carried state), and leaves S, the segment's decay and for an mLSTM n and m in a SegEntry; the second
-// (SEG_FULL) starts every segment from the entries before it, folded in order. The state half is under half of the work of a chunk.
-// One prompt of 8192 tokens: 64 heads of 128 x 64 (128 CTAs, 2 segments) and 16 heads of 128 x 128 (64 CTAs, 4 segments) took 408 us on
-// average, now 270 in both launches together.
+// cut into segments of whole chunks: a first launch (SEG_STATE) runs the state half alone, one chain over every segment but the
+// last, and leaves the state before each segment in a SegEntry; the second (SEG_FULL) runs all segments side by side from
+// there. The chain has the products and sums of the form without segments, in their order, so the results are the same bit by bit.
+// (Segments that each start from zero and are folded with their decays shorten the chain, but round in another order.) The state half is
+// under half of the work of a chunk, and the chain has its eight warps to itself: half of the columns each, a ninth prepares the vectors.
+// One prompt of 8192 tokens, 16 heads of 128 x 128 (64 CTAs, 4 segments): 324 -> 228 us in both launches together; a chunk costs the
+// chain 1.0 us, the whole form 2.5.
 constexpr int WHOLE = 0, SEG_STATE = 1, SEG_FULL = 2;
 constexpr int CQ = 64, CP = 32, CPP = CP + 8;
-template <int NT>
-struct ChunkSmem {
-  static constexpr int NP = NT + 8;
-  static constexpr int QK = CQ * NP * 2, V = CQ * CPP * 2, STAGE = 2 * QK + V;          // bytes
-  static constexpr int W = 2 * STAGE, S = W + 2 * V, VEC = S + 2 * NT * CPP * 2, VECS = 6 * CQ, NB = VEC + 2 * VECS * 4;
+template <int NT, int MODE>
+struct ChunkSmem {                                               // a stage holds q (not in the chain of SEG_STATE), k and v of a chunk
+  static constexpr int NP = NT + 8, STAGES = MODE == SEG_STATE ? 4 : 2;
+  static constexpr int QK = CQ * NP * 2, V = CQ * CPP * 2, K_AT = MODE == SEG_STATE ? 0 : QK, V_AT = K_AT + QK, STAGE = V_AT + V;          // bytes
+  static constexpr int W = STAGES * STAGE, S = W + 2 * V, VEC = S + (MODE == SEG_STATE ? 0 : 2 * NT * CPP * 2), VECS = 6 * CQ, NB = VEC + 2 * VECS * 4;
   static constexpr int BYTES = NB, BYTES_ML = NB + 2 * NT * 2;     // mLSTM: n as hi, lo
 };
 struct ChunkVec {                                                // one chunk's vectors, 64 each
   float *L, *step, *E, *F;                                       // L; d; 2^(L_63 - L_s) d; 2^(L_e - L_s) d, e = end of s's 16-block
   float *floor, *m;                                              // mLSTM: exp(-m_t); m before the chunk. L = -A, step = a
 };
-// What a segment leaves for those after it, fp32: S [NT][32], n [NT], {log2 of its decay, m in log2}. The entry of a sequence's last
-// segment holds the state that the sequence brought: nothing may read p.state in the second launch, which renews it.
+// The state after a segment as the registers hold it, fp32: S [NT][32], n [NT][2] (its hi and lo column), m in log2. The entry of a
+// sequence's last segment holds the state that the sequence brought: nothing may read p.state in the second launch, which renews it.
 template <int NT>
-struct SegEntry { static constexpr int N = NT * CP, LOG = N + NT, FLOATS = LOG + 4; };
+struct SegEntry { static constexpr int N = NT * CP, M = N + 2 * NT, FLOATS = M + 4; };
+constexpr int chunk_threads(int mode) { return mode == SEG_STATE ? 288 : 256; }
 template <int NT, bool ML, int MODE>
-__global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(const ScanParams p, int slices, int conv_parts) {
-  using L = ChunkSmem<NT>;
+__global__ void __launch_bounds__(chunk_threads(MODE), NT <= 128 ? 2 : 1) scan_chunk_kernel(const ScanParams p, int slices, int conv_parts) {
+  using L = ChunkSmem<NT, MODE>;
   using bf16 = __nv_bfloat16;
-  const int sq = MODE == WHOLE ? blockIdx.z : blockIdx.z / p.segs, seg = MODE == WHOLE ? 0 : blockIdx.z - sq * p.segs, s = p.seq0 + sq;
+  const int sq = MODE == SEG_FULL ? blockIdx.z / p.segs : blockIdx.z, seg = MODE == SEG_FULL ? blockIdx.z - sq * p.segs : 0, s = p.seq0 + sq;
   if ((int)blockIdx.x >= slices) {
     if (blockIdx.y == 0 && seg == 0) conv_tail<bf16>(p, s, blockIdx.x - slices, conv_parts);
     return;
@@ -425,8 +428,9 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
   const int c0 = blockIdx.x * CP, ncol = min(CP, p.P - c0), grp = h / p.rep;
   const int slot = p.sslot[s];
   const int last_seg = MODE == WHOLE ? 0 : min((n - 1) / p.seg_len, p.segs - 1);       // the tokens [tb, te) are this CTA's
-  if (MODE != WHOLE && (n <= 0 || seg > last_seg || (MODE == SEG_STATE && seg == last_seg))) return;
-  const int tb = MODE == WHOLE ? 0 : seg * p.seg_len, te = seg == last_seg ? n : tb + p.seg_len;
+  if (MODE != WHOLE && (n <= 0 || seg > last_seg || (MODE == SEG_STATE && last_seg == 0))) return;
+  const int tb = MODE == SEG_FULL ? seg * p.seg_len : 0;
+  const int te = MODE == SEG_STATE ? last_seg * p.seg_len : (seg == last_seg ? n : tb + p.seg_len);
   auto entry = [&](int i) { return p.seg_ws + ((((long long)sq * p.segs + i) * p.heads + h) * slices + blockIdx.x) * SegEntry<NT>::FLOATS; };
   const bf16* q = reinterpret_cast<const bf16*>(p.q) + row0 * p.q_ld + (long long)grp * p.N;
   const bf16* k = reinterpret_cast<const bf16*>(p.k) + row0 * p.k_ld + (long long)grp * p.N;
@@ -437,6 +441,7 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
     return ChunkVec{f, f + CQ, f + 2 * CQ, f + 3 * CQ, f + 4 * CQ, f + 5 * CQ};
   };
   auto load = [&](int stage, int t0) {
+    if (MODE == SEG_STATE && warp == 8) return;
     constexpr int STEP = 256 / (NT / 8);                         // rows per pass
     const uint32_t base = sb + stage * L::STAGE;
     const int r0 = threadIdx.x / (NT / 8), c = threadIdx.x % (NT / 8);
@@ -448,16 +453,22 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
     for (int i = 0; i < CQ / STEP; ++i) {
       const bool ok = cok && t0 + r0 + i * STEP < n;
       if (MODE != SEG_STATE) cp_async16(dst + i * STEP * L::NP * 2, ok ? qp : q, ok);
-      cp_async16(dst + i * STEP * L::NP * 2 + L::QK, ok ? kp : k, ok);
+      cp_async16(dst + i * STEP * L::NP * 2 + L::K_AT, ok ? kp : k, ok);
       qp += STEP * p.q_ld;
       kp += STEP * p.k_ld;
     }
     const int r = threadIdx.x / (CP / 8), cv = threadIdx.x % (CP / 8);     // 64 rows x 4 pieces
     const bool ok = t0 + r < n && cv * 8 < ncol;
-    cp_async16(base + 2 * L::QK + (r * CPP + cv * 8) * 2, ok ? v + (t0 + r) * p.v_ld + cv * 8 : v, ok);
+    cp_async16(base + L::V_AT + (r * CPP + cv * 8) * 2, ok ? v + (t0 + r) * p.v_ld + cv * 8 : v, ok);
     cp_async_commit();
   };
-  load(0, tb);
+  // every chunk commits one group, also where nothing is left to load
+  auto load_ahead = [&](int it, int t0) {
+    if (t0 + (L::STAGES - 1) * CQ < te) load((it + L::STAGES - 1) & (L::STAGES - 1), t0 + (L::STAGES - 1) * CQ);
+    else cp_async_commit();
+  };
+#pragma unroll
+  for (int i = 0; i < L::STAGES - 1; ++i) load_ahead(i - (L::STAGES - 1), tb + (i - (L::STAGES - 1)) * CQ);
 
   const bool have = slot >= 0 && start > 0;
   constexpr float LOG2E = 1.4426950408889634f;
@@ -466,7 +477,6 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
   const float bias = ML ? p.gate_b[h] : (p.decay ? 0.f : p.dt_bias[h]);
   const float bias_f = ML ? p.gate_b[p.heads + h] : 0.f;
   float* vecs = ML ? p.vec + (((long long)(slot < 0 ? 0 : slot) * p.heads + h) * slices + blockIdx.x) * (p.N + 1) : nullptr;
-  float logs = 0.f;                                              // warp PREP: log2 of the decay of the chunks prepared so far
   float m = 0.f;                                                 // warp PREP, mLSTM: log2 of the running maximum
   // warp PREP: step sizes and decays of the chunk at t0, two consecutive tokens a lane
   auto raw_dt = [&](int t0, float (&d)[4]) {                     // mLSTM: input gates, then forget gates
@@ -511,9 +521,7 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
     *reinterpret_cast<float2*>(cv.F + 2 * lane) = make_float2(ex2(a[0] - Ae), ex2(a[1] - Ae));
     *reinterpret_cast<float2*>(cv.floor + 2 * lane) = make_float2(ex2(-(F0 + A0)), ex2(-(F1 + A1)));
     if (lane == 0) *cv.m = m;
-    const float F = __shfl_sync(0xffffffffu, F1, 31);
-    logs += F;
-    m = F + last;
+    m = __shfl_sync(0xffffffffu, F1, 31) + last;
   };
   auto prepare = [&](int i, int t0, const float (&d)[4]) {
     float step[2], l[2];
@@ -532,7 +540,6 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
     }
     const float before = x - l[1];
     const float total = __shfl_sync(0xffffffffu, x, 31);
-    logs += total;
     const float le = __shfl_sync(0xffffffffu, x, lane | 7);      // end of this 16-token block
     const float l0 = before + l[0], l1 = x;
     const ChunkVec cv = vec(i);
@@ -541,29 +548,14 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
     *reinterpret_cast<float2*>(cv.E + 2 * lane) = make_float2(ex2(total - l0) * step[0], ex2(total - l1) * step[1]);
     *reinterpret_cast<float2*>(cv.F + 2 * lane) = make_float2(ex2(le - l0) * step[0], ex2(le - l1) * step[1]);
   };
-  auto fold_m = [&](int i, float& m, float& keep, float& gain) {  // the entry of segment i behind a maximum m: factors of old and new
-    const float *e = entry(i) + SegEntry<NT>::LOG, F = e[0], mi = e[1], x = fmaxf(F + m, mi);
-    keep = ex2(F + m - x);
-    gain = ex2(mi - x);
-    m = x;
-  };
   float d[4] = {0.f, 0.f, 0.f, 0.f};
   // the warp that prepares the vectors: see above; the gates of an mLSTM are more than the slack of warp 0
-  constexpr int PREP = ML && MODE != SEG_STATE ? 4 : 0;
+  constexpr int PREP = MODE == SEG_STATE ? 8 : (ML ? 4 : 0);
   if (warp == PREP) {
     if constexpr (ML) {
-      if (MODE == SEG_FULL && seg > 0) {
-        m = entry(0)[SegEntry<NT>::LOG + 1];
-        float keep, gain;
-        for (int i = 1; i < seg; ++i) fold_m(i, m, keep, gain);
-      } else if (MODE == SEG_FULL && last_seg > 0) {
-        m = entry(last_seg)[SegEntry<NT>::LOG + 1];
-      } else if (MODE == SEG_STATE && seg > 0) {
-        m = -INFINITY;
-      } else if (have) {
-        m = vecs[p.N] * LOG2E;
-      }
-      if (MODE == SEG_STATE && seg == 0 && lane == 0) entry(last_seg)[SegEntry<NT>::LOG + 1] = m;
+      if (MODE == SEG_FULL && last_seg > 0) m = entry(seg > 0 ? seg - 1 : last_seg)[SegEntry<NT>::M];
+      else if (have) m = vecs[p.N] * LOG2E;
+      if (MODE == SEG_STATE && lane == 0) entry(last_seg)[SegEntry<NT>::M] = m;
     }
     raw_dt(tb, d);
     if constexpr (ML) prepare_ml(0, tb, d);
@@ -577,29 +569,27 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
     raw_dt(t0 + 2 * CQ, d);
   };
 
-  if (MODE == SEG_STATE && warp < 4) {
-    int it = 0;
+  if (MODE == SEG_STATE && warp == PREP) {
+    int it = 0, ends = p.seg_len, i = 0;                         // end and number of the segment
     for (int t0 = tb; t0 < te; t0 += CQ, ++it) {
-      cp_async_wait<0>();
       __syncthreads();
-      if (t0 + CQ < te) load((it + 1) & 1, t0 + CQ);
+      if (t0 + CQ == ends) {
+        if (ML && lane == 0) entry(i)[SegEntry<NT>::M] = m;
+        ends += p.seg_len;
+        ++i;
+      }
       prepare_next(it, t0);
-    }
-    if (warp == 0 && lane == 0) {
-      float* e = entry(seg) + SegEntry<NT>::LOG;
-      e[0] = logs;
-      e[1] = m;
     }
     return;
   }
-  if (warp < 4) {
+  if (MODE != SEG_STATE && warp < 4) {
     // ---- outputs of 16 tokens per chunk ----
     const int scol = (lane & 3) * 2, tr = warp * 16 + (lane >> 2);
     int it = 0;
     for (int t0 = tb; t0 < te; t0 += CQ, ++it) {
-      cp_async_wait<0>();
+      cp_async_wait<L::STAGES - 2>();
       __syncthreads();                                           // tile, vectors and S operand of this chunk are there
-      if (t0 + CQ < te) load((it + 1) & 1, t0 + CQ);
+      load_ahead(it, t0);
       const uint32_t base = sb + (it & 1) * L::STAGE;
       const ChunkVec cv = vec(it);
       uint32_t qf[NT / 16][4];
@@ -696,7 +686,7 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
           mma_bf16(o[2 * j + 1], lo, b[2], b[3]);
         }
       }
-      const bf16* sv = reinterpret_cast<const bf16*>(smem + (it & 1) * L::STAGE + 2 * L::QK);
+      const bf16* sv = reinterpret_cast<const bf16*>(smem + (it & (L::STAGES - 1)) * L::STAGE + L::V_AT);
 #pragma unroll
       for (int y = 0; y < 2; ++y) {
         const int t = tr + 8 * y;
@@ -725,11 +715,13 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
   }
 
   // ---- state ----
-  const int sw = warp - 4;
+  // NT / 4 rows a warp, in the chain of SEG_STATE half of the columns
+  constexpr int STATE_THREADS = MODE == SEG_STATE ? 256 : 128, JN = MODE == SEG_STATE ? 1 : 2;     // JN: groups of 16 columns
+  const int sw = MODE == SEG_STATE ? warp & 3 : warp - 4, jc = MODE == SEG_STATE ? (warp >> 2) * 16 : 0;
   constexpr int MT = NT / 64;                                    // 16-row state tiles of a warp
-  float S[MT][CP / 8][4];
+  float S[MT][2 * JN][4];
   float* st = p.state + (((long long)(slot < 0 ? 0 : slot) * p.heads + h) * p.N) * p.P + c0;
-  const int srow = sw * (NT / 4) + (lane >> 2), scol = (lane & 3) * 2;
+  const int srow = sw * (NT / 4) + (lane >> 2), scol = (lane & 3) * 2, col0 = jc + scol;
   float ns[ML ? MT : 1][4];                                      // mLSTM: columns 0 (from hi) and 1 (from lo) in lanes 4 r; n is their sum
   auto publish = [&]() {                                         // S as hi / lo operands
     if constexpr (ML) {
@@ -748,24 +740,24 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
-      for (int j = 0; j < CP / 8; ++j)
+      for (int j = 0; j < 2 * JN; ++j)
 #pragma unroll
         for (int y = 0; y < 2; ++y) {
           uint32_t hi, lo;
           split_pair(S[i][j][2 * y], S[i][j][2 * y + 1], hi, lo);
-          const int off = ((srow + i * 16 + 8 * y) * CPP + j * 8 + scol) * 2;
+          const int off = ((srow + i * 16 + 8 * y) * CPP + j * 8 + col0) * 2;
           *reinterpret_cast<uint32_t*>(smem + L::S + off) = hi;
           *reinterpret_cast<uint32_t*>(smem + L::S + NT * CPP * 2 + off) = lo;
         }
   };
-  // the state before the segment: carried, from zero, or the entries of the segments before it
+  // the state before the segment: carried, or the entry of the segment before it
   auto each = [&](auto f) {
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
-      for (int j = 0; j < CP / 8; ++j)
+      for (int j = 0; j < 2 * JN; ++j)
 #pragma unroll
-        for (int x = 0; x < 4; ++x) f(S[i][j][x], srow + i * 16 + 8 * (x >> 1), j * 8 + scol + (x & 1));
+        for (int x = 0; x < 4; ++x) f(S[i][j][x], srow + i * 16 + 8 * (x >> 1), j * 8 + col0 + (x & 1));
   };
   auto each_n = [&](auto f) {
     if constexpr (ML)
@@ -774,41 +766,38 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
 #pragma unroll
         for (int y = 0; y < 2; ++y) f(ns[i][2 * y], ns[i][2 * y + 1], srow + i * 16 + 8 * y);
   };
+  auto save = [&](int i) {
+    float* e = entry(i);
+    each([&](float& x, int r, int c) { e[r * CP + c] = x; });
+    each_n([&](float& a, float& b, int r) {
+      if ((lane & 3) == 0 && jc == 0) *reinterpret_cast<float2*>(e + SegEntry<NT>::N + 2 * r) = make_float2(a, b);
+    });
+  };
   if (MODE == SEG_FULL && last_seg > 0) {
-    const float* e = entry(seg > 0 ? 0 : last_seg);
+    const float* e = entry(seg > 0 ? seg - 1 : last_seg);
     each([&](float& x, int r, int c) { x = e[r * CP + c]; });
-    each_n([&](float& a, float& b, int r) { a = (lane & 3) == 0 ? e[SegEntry<NT>::N + r] : 0.f; b = 0.f; });
-    float mm = ML && seg > 0 ? e[SegEntry<NT>::LOG + 1] : 0.f;
-    for (int i = 1; i < seg; ++i) {
-      const float* ei = entry(i);
-      float keep, gain = 1.f;
-      if constexpr (ML) fold_m(i, mm, keep, gain);
-      else keep = ex2(ei[SegEntry<NT>::LOG]);
-      each([&](float& x, int r, int c) { x = fmaf(keep, x, gain * ei[r * CP + c]); });
-      each_n([&](float& a, float&, int r) { if ((lane & 3) == 0) a = fmaf(keep, a, gain * ei[SegEntry<NT>::N + r]); });
-    }
+    each_n([&](float& a, float& b, int r) {
+      const float2 u = (lane & 3) == 0 ? *reinterpret_cast<const float2*>(e + SegEntry<NT>::N + 2 * r) : make_float2(0.f, 0.f);
+      a = u.x;
+      b = u.y;
+    });
   } else {
-    const bool carried = have && (MODE != SEG_STATE || seg == 0);
-    each([&](float& x, int r, int c) { x = carried && r < p.N && c < ncol ? st[(long long)r * p.P + c] : 0.f; });
-    each_n([&](float& a, float& b, int r) { a = carried && (lane & 3) == 0 && r < p.N ? vecs[r] : 0.f; b = 0.f; });
-    if (MODE == SEG_STATE && seg == 0) {
-      float* e = entry(last_seg);
-      each([&](float& x, int r, int c) { e[r * CP + c] = x; });
-      each_n([&](float& a, float&, int r) { if ((lane & 3) == 0) e[SegEntry<NT>::N + r] = a; });
-    }
+    each([&](float& x, int r, int c) { x = have && r < p.N && c < ncol ? st[(long long)r * p.P + c] : 0.f; });
+    each_n([&](float& a, float& b, int r) { a = have && (lane & 3) == 0 && r < p.N ? vecs[r] : 0.f; b = 0.f; });
+    if (MODE == SEG_STATE) save(last_seg);
   }
   if (MODE != SEG_STATE) publish();
-  int it = 0;
+  int it = 0, ends = p.seg_len, seg_i = 0;                       // SEG_STATE: end and number of the segment
   for (int t0 = tb; t0 < te; t0 += CQ, ++it) {
-    cp_async_wait<0>();
+    cp_async_wait<L::STAGES - 2>();
     __syncthreads();
-    if (t0 + CQ < te) load((it + 1) & 1, t0 + CQ);
-    const uint32_t base = sb + (it & 1) * L::STAGE;
+    load_ahead(it, t0);
+    const uint32_t base = sb + (it & (L::STAGES - 1)) * L::STAGE;
     const ChunkVec cv = vec(it);
-    const bf16* sv = reinterpret_cast<const bf16*>(smem + (it & 1) * L::STAGE + 2 * L::QK);
+    const bf16* sv = reinterpret_cast<const bf16*>(smem + (it & (L::STAGES - 1)) * L::STAGE + L::V_AT);
 #pragma unroll
-    for (int i = 0; i < CQ * CP / 2 / 128; ++i) {                // scaled values as hi / lo operands
-      const int r = (threadIdx.x - 128) / (CP / 2) + i * (128 / (CP / 2)), c = 2 * (threadIdx.x % (CP / 2));
+    for (int i = 0; i < CQ * CP / 2 / STATE_THREADS; ++i) {      // scaled values as hi / lo operands
+      const int r = (threadIdx.x & (STATE_THREADS - 1)) / (CP / 2) + i * (STATE_THREADS / (CP / 2)), c = 2 * (threadIdx.x % (CP / 2));
       const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sv + r * CPP + c));
       const float e = cv.E[r];
       uint32_t hi, lo;
@@ -820,22 +809,22 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
 #pragma unroll
     for (int i = 0; i < MT; ++i) {
 #pragma unroll
-      for (int j = 0; j < CP / 8; ++j)
+      for (int j = 0; j < 2 * JN; ++j)
 #pragma unroll
         for (int x = 0; x < 4; ++x) S[i][j][x] *= keep;
       if constexpr (ML)
 #pragma unroll
         for (int x = 0; x < 4; ++x) ns[i][x] *= keep;
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");               // scaled values written (warps 4-7)
+    asm volatile("bar.sync 1, %0;" ::"n"(STATE_THREADS) : "memory");       // scaled values written
 #pragma unroll
     for (int kb = 0; kb < CQ / 16; ++kb) {
-      uint32_t w[2][CP / 16][4];
-      const uint32_t wa = sb + L::W + ((kb * 16 + (lane & 15)) * CPP + (lane >> 4) * 8) * 2;
+      uint32_t w[2][JN][4];
+      const uint32_t wa = sb + L::W + ((kb * 16 + (lane & 15)) * CPP + jc + (lane >> 4) * 8) * 2;
 #pragma unroll
       for (int x = 0; x < 2; ++x)
 #pragma unroll
-        for (int j = 0; j < CP / 16; ++j) ldsm4_t(w[x][j], wa + x * L::V + j * 32);
+        for (int j = 0; j < JN; ++j) ldsm4_t(w[x][j], wa + x * L::V + j * 32);
       uint32_t e0 = 0, e1 = 0;                                   // mLSTM: factors of keys 16 kb .. as columns 0 (hi) and 1 (lo)
       if constexpr (ML) {
         const float2 u = *reinterpret_cast<const float2*>(cv.E + kb * 16 + scol), v2 = *reinterpret_cast<const float2*>(cv.E + kb * 16 + 8 + scol);
@@ -848,34 +837,36 @@ __global__ void __launch_bounds__(256, NT <= 128 ? 2 : 1) scan_chunk_kernel(cons
       for (int i = 0; i < MT; ++i) {
         // A = K^T: rows n, columns s, read transposed from K [s][n]
         uint32_t a[4];
-        ldsm4_t(a, base + L::QK + ((kb * 16 + (lane & 7) + ((lane >> 4) << 3)) * L::NP + sw * (NT / 4) + i * 16 + ((lane >> 3) & 1) * 8) * 2);
+        ldsm4_t(a, base + L::K_AT + ((kb * 16 + (lane & 7) + ((lane >> 4) << 3)) * L::NP + sw * (NT / 4) + i * 16 + ((lane >> 3) & 1) * 8) * 2);
 #pragma unroll
         for (int x = 0; x < 2; ++x)
 #pragma unroll
-          for (int j = 0; j < CP / 16; ++j) {
+          for (int j = 0; j < JN; ++j) {
             mma_bf16(S[i][2 * j], a, w[x][j][0], w[x][j][1]);
             mma_bf16(S[i][2 * j + 1], a, w[x][j][2], w[x][j][3]);
           }
         if constexpr (ML) mma_bf16(ns[i], a, e0, e1);
       }
     }
-    if (MODE == SEG_STATE) continue;
+    if (MODE == SEG_STATE) {
+      if (t0 + CQ == ends) {
+        save(seg_i++);
+        ends += p.seg_len;
+      }
+      continue;
+    }
     prepare_next(it, t0);
     asm volatile("bar.sync 2, 256;" ::: "memory");               // warps 0-3 have read the old operand
     publish();
   }
-  if (MODE == SEG_STATE) {
-    float* e = entry(seg);
-    each([&](float& x, int r, int c) { e[r * CP + c] = x; });
-    each_n([&](float& a, float& b, int r) { if ((lane & 3) == 0) e[SegEntry<NT>::N + r] = a + b; });
-  } else if (slot >= 0 && seg == last_seg) {
+  if (MODE != SEG_STATE && slot >= 0 && seg == last_seg) {
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
-      for (int j = 0; j < CP / 8; ++j)
+      for (int j = 0; j < 2 * JN; ++j)
 #pragma unroll
         for (int y = 0; y < 2; ++y) {
-          const int r = srow + i * 16 + 8 * y, c = j * 8 + scol;
+          const int r = srow + i * 16 + 8 * y, c = j * 8 + col0;
           if (r < p.N && c < ncol) {
             st[(long long)r * p.P + c] = S[i][j][2 * y];
             st[(long long)r * p.P + c + 1] = S[i][j][2 * y + 1];
@@ -906,7 +897,7 @@ inline int scan_segments(int longest, int nseq, int heads, int P) {
 template <int NT, bool ML, int MODE>
 int launch_chunk_mode(const ScanParams& p, int nseq, int conv_parts, cudaStream_t st) {
   static bool done[64] = {};
-  const int bytes = ML ? ChunkSmem<NT>::BYTES_ML : ChunkSmem<NT>::BYTES;
+  const int bytes = ML ? ChunkSmem<NT, MODE>::BYTES_ML : ChunkSmem<NT, MODE>::BYTES;
   int dev = 0;
   DLTI_CUDA_CHECK(cudaGetDevice(&dev));
   if (!done[dev & 63]) {
@@ -914,7 +905,7 @@ int launch_chunk_mode(const ScanParams& p, int nseq, int conv_parts, cudaStream_
     done[dev & 63] = true;
   }
   const int slices = (p.P + CP - 1) / CP;
-  scan_chunk_kernel<NT, ML, MODE><<<dim3(slices + conv_parts, p.heads, nseq * (MODE == WHOLE ? 1 : p.segs)), 256, bytes, st>>>(p, slices, conv_parts);
+  scan_chunk_kernel<NT, ML, MODE><<<dim3(slices + conv_parts, p.heads, nseq * (MODE == SEG_FULL ? p.segs : 1)), chunk_threads(MODE), bytes, st>>>(p, slices, conv_parts);
   dlti_count_launch();
   return (int)cudaGetLastError();
 }
