@@ -886,12 +886,18 @@ __global__ void __launch_bounds__(chunk_threads(MODE), NT <= 128 ? 2 : 1) scan_c
   }
 }
 
-// Segments per sequence: as many as give the SMs two CTAs each, of at least 8 chunks, where there is room for two or more.
-inline int scan_segments(int longest, int nseq, int heads, int P) {
-  const long long ctas = (long long)((P + CP - 1) / CP) * heads * nseq, room = 2LL * dlti_num_sms() / (ctas > 0 ? ctas : 1);
+// Segments per sequence: as many as fill the SMs with the CTAs that fit one of them side by side (two up to 128 rows of a state, one
+// above: shared memory), of at least 8 chunks. Two CTAs of an SM slow each other down, so that more than one per SM has to come with
+// three segments or more. 8192 tokens in 1 / 2 / 3 / 4 / 8 segments, us, heads of 128 x 128: 32 CTAs 339 / 243 / 208 / 189 / 185, 64 CTAs 341 /
+// 247 / 263 / 230 / 253, 96 CTAs 344 / 329 / 267 / 359 / 321, 128 CTAs 343 / 327 / 431 / 364 / 386 and, where a step size is computed, 354 / 353
+// / 460; 1024 tokens of 128 CTAs: 52 whole, 60 in two. Heads of 256 x 256, 4096 tokens: 64 CTAs 266 / 192 / 251, 96 CTAs 267 / 325 / 261.
+inline int scan_segments(int longest, int nseq, int heads, int N, int P) {
+  const long long ctas = (long long)((P + CP - 1) / CP) * heads * nseq, sms = dlti_num_sms();
+  const long long room = (N <= 128 ? 2 : 1) * sms / (ctas > 0 ? ctas : 1);
   const int most = longest / (8 * CQ);
-  const int segs = (int)(room < most ? room : most);
-  return segs > 1 ? (segs < 16 ? segs : 16) : 1;
+  int segs = (int)(room < most ? room : most);
+  segs = segs < 16 ? segs : 16;
+  return segs > 2 || (segs == 2 && 2 * ctas <= sms) ? segs : 1;
 }
 
 template <int NT, bool ML, int MODE>
@@ -919,7 +925,7 @@ int launch_chunk(const ScanParams& p, int nseq, cudaStream_t st) {
 inline int segment_floats(int N) { return N <= 64 ? SegEntry<64>::FLOATS : (N <= 128 ? SegEntry<128>::FLOATS : SegEntry<256>::FLOATS); }
 // segments of at most `longest` rows a sequence in ws (null: none)
 inline void set_segments(ScanParams& p, int longest, int nseq, float* ws) {
-  const int segs = ws ? scan_segments(longest, nseq, p.heads, p.P) : 1;
+  const int segs = ws ? scan_segments(longest, nseq, p.heads, p.N, p.P) : 1;
   if (segs <= 1 || (long long)nseq * segs > 65535) return;
   p.seg_len = ((longest + segs - 1) / segs + CQ - 1) / CQ * CQ;
   p.segs = (longest + p.seg_len - 1) / p.seg_len;
@@ -1010,7 +1016,7 @@ DLTI_API int dlti_linear_scan_chunked(const void* q, long long q_ld, const void*
 // floats of workspace with which the chunked forms cut sequences of up to `longest` rows into segments (0: they would not)
 DLTI_API long long dlti_scan_workspace(int longest, int nseq, int heads, int N, int P) {
   if (nseq < 1 || heads < 1 || P < 1 || N < 1 || N > 256) return 0;
-  const int segs = scan_segments(longest, nseq, heads, P);
+  const int segs = scan_segments(longest, nseq, heads, N, P);
   return segs > 1 ? (long long)nseq * segs * heads * ((P + CP - 1) / CP) * segment_floats(N) : 0;
 }
 
