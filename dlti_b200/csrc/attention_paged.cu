@@ -9,8 +9,8 @@
 //                        results through shared memory, more leave them to attn_combine_kernel
 //   attn_rows_kernel     one warp per (row, head), fp32 arithmetic throughout: the fp32 mode, and heads above 256
 //
-// Scores, softmax weights and sums are fp32. The weights enter the P*V product as two 16-bit terms (hi + lo, 16 mantissa
-// bits and more), so the product is that of the fp32 weights with the 16-bit values.
+// Scores, softmax weights and sums are fp32. The weights enter the P*V product as two bf16 terms (hi + lo, 16 mantissa bits); for
+// Llama (dlti_paged_decode_groups) as three, which hold all of their 24 bits.
 #include "mma_sync.cuh"
 #include "pair.cuh"
 #include "rows.cuh"
@@ -218,24 +218,54 @@ __device__ __forceinline__ void scores16(float (&s0)[4], float (&s1)[4], const u
     mma_16<T>(s1, qf[kk], b[2], b[3]);
   }
 }
-// O += P[16 x 16 keys] V, the weights as hi + lo
-template <int DV, typename T = bf16>
-__device__ __forceinline__ void weighted16(float (&o)[DV / 8][4], const float (&p0)[4], const float (&p1)[4], uint32_t v_base, int kt) {
+// O += P[16 x 16 keys] V, the weights as three terms. An infinite value stays what it is in the product with the first one, as in a
+// product of fp32 numbers (weights below 2^-33 of the largest are zero in fp16); NaNs too: min and max drop them from the other two alone.
+template <int DV, typename T>
+__device__ __forceinline__ void weighted16_full(float (&o)[DV / 8][4], const float (&p0)[4], const float (&p1)[4], uint32_t v_base, int kt) {
   const int lane = threadIdx.x & 31;
-  uint32_t hi[4], lo[4];
-  split_pair_16<T>(p0[0], p0[1], hi[0], lo[0]);
-  split_pair_16<T>(p0[2], p0[3], hi[1], lo[1]);
-  split_pair_16<T>(p1[0], p1[1], hi[2], lo[2]);
-  split_pair_16<T>(p1[2], p1[3], hi[3], lo[3]);
+  uint32_t w[4][3], a[3][4];
+  split3_pair_16<T>(p0[0], p0[1], w[0]);
+  split3_pair_16<T>(p0[2], p0[3], w[1]);
+  split3_pair_16<T>(p1[0], p1[1], w[2]);
+  split3_pair_16<T>(p1[2], p1[3], w[3]);
+#pragma unroll
+  for (int t = 0; t < 3; ++t)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) a[t][x] = w[x][t];
   const uint32_t addr = v_base + ((kt + (lane & 15)) * (DV + 8) + (lane >> 4) * 8) * 2;
 #pragma unroll
   for (int d = 0; d < DV / 16; ++d) {
     uint32_t b[4];
     ldsm4_t(b, addr + d * 32);
-    mma_16<T>(o[2 * d], hi, b[0], b[1]);
-    mma_16<T>(o[2 * d], lo, b[0], b[1]);
-    mma_16<T>(o[2 * d + 1], hi, b[2], b[3]);
-    mma_16<T>(o[2 * d + 1], lo, b[2], b[3]);
+    mma_16<T>(o[2 * d], a[0], b[0], b[1]);
+    mma_16<T>(o[2 * d + 1], a[0], b[2], b[3]);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) b[x] = finite_pair_16<T>(b[x]);
+#pragma unroll
+    for (int t = 1; t < 3; ++t) {
+      mma_16<T>(o[2 * d], a[t], b[0], b[1]);
+      mma_16<T>(o[2 * d + 1], a[t], b[2], b[3]);
+    }
+  }
+}
+// O += P[16 x 16 keys] V, the weights as hi + lo
+template <int DV>
+__device__ __forceinline__ void weighted16(float (&o)[DV / 8][4], const float (&p0)[4], const float (&p1)[4], uint32_t v_base, int kt) {
+  const int lane = threadIdx.x & 31;
+  uint32_t hi[4], lo[4];
+  split_pair(p0[0], p0[1], hi[0], lo[0]);
+  split_pair(p0[2], p0[3], hi[1], lo[1]);
+  split_pair(p1[0], p1[1], hi[2], lo[2]);
+  split_pair(p1[2], p1[3], hi[3], lo[3]);
+  const uint32_t addr = v_base + ((kt + (lane & 15)) * (DV + 8) + (lane >> 4) * 8) * 2;
+#pragma unroll
+  for (int d = 0; d < DV / 16; ++d) {
+    uint32_t b[4];
+    ldsm4_t(b, addr + d * 32);
+    mma_bf16(o[2 * d], hi, b[0], b[1]);
+    mma_bf16(o[2 * d], lo, b[0], b[1]);
+    mma_bf16(o[2 * d + 1], hi, b[2], b[3]);
+    mma_bf16(o[2 * d + 1], lo, b[2], b[3]);
   }
 }
 
@@ -400,7 +430,7 @@ __device__ __forceinline__ float ld_peer_f32(uint32_t addr, uint32_t rank) {
 // chain of latencies (context length, page table, keys, products, merge), so what counts is the number of steps and launches:
 // CLUSTER: the splits of a head are one cluster, whose CTAs merge each a part of the columns, in the place of a second kernel.
 // fp16 weights are scaled by 2^8 against their subnormals; it cancels in the division.
-template <typename T, int DK, int DV, bool CLUSTER>
+template <typename T, int DK, int DV, bool CLUSTER, bool FULL>      // FULL: weights of 24 bits
 __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, int splits, float* __restrict__ part_o,
                                                          float* __restrict__ part_ml) {
   using L = Tile<DK, DV>;
@@ -483,7 +513,8 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, i
           s[i][x] = ex2(s[i][x] - m[x >> 1] + LIFT);
           l[x >> 1] += s[i][x];
         }
-      weighted16<DV, T>(o, s[0], s[1], vb, warp * 16);
+      if constexpr (FULL) weighted16_full<DV, T>(o, s[0], s[1], vb, warp * 16);
+      else weighted16<DV>(o, s[0], s[1], vb, warp * 16);
     }
   }
   // merge the four warps; the stages are free after the barrier
@@ -622,12 +653,12 @@ int launch_prefill(const PagedParams& p, int nseq, int max_rows, cudaStream_t st
   return (int)cudaGetLastError();
 }
 
-template <typename T, int DK, int DV>
+template <typename T, int DK, int DV, bool FULL = false>
 int launch_decode_t(const PagedParams& p, int splits, float* ws, cudaStream_t st) {
   static bool done[2][64] = {};
   constexpr int merge = 5 * 16 * DV * 4, tiles = 2 * Tile<DK, DV>::BYTES, smem = tiles > merge ? tiles : merge;
   const bool cluster = splits > 1 && splits <= 8;
-  auto kern = cluster ? attn_decode_kernel<T, DK, DV, true> : attn_decode_kernel<T, DK, DV, false>;
+  auto kern = cluster ? attn_decode_kernel<T, DK, DV, true, FULL> : attn_decode_kernel<T, DK, DV, false, FULL>;
   if (int rc = allow_smem(kern, smem, done[cluster])) return rc;
   const int rep = p.H / p.G;
   float* part_ml = cluster ? nullptr : ws + (long long)p.rows * p.H * splits * p.vdim;
@@ -719,7 +750,7 @@ int dlti_paged_decode_groups(const void* q, long long q_ld, const void* kc, cons
                              cudaStream_t st) {
   PagedParams p{q, q_ld, 128, kc, vc, 128, 128, tables, max_blocks, bs, ctx, nullptr, nullptr, nullptr, 0, H, G, 128, 128, 0, 0, scale, 0.f,
                 nullptr, out, o_ld, batch, nullptr, nullptr, 0, nullptr, 0};
-  if (dtype == DLTI_BF16) return launch_decode_t<bf16, 128, 128>(p, splits, ws, st);
-  if (dtype == DLTI_FP16) return launch_decode_t<__half, 128, 128>(p, splits, ws, st);
+  if (dtype == DLTI_BF16) return launch_decode_t<bf16, 128, 128, true>(p, splits, ws, st);
+  if (dtype == DLTI_FP16) return launch_decode_t<__half, 128, 128, true>(p, splits, ws, st);
   return DLTI_ERR_UNSUPPORTED;
 }

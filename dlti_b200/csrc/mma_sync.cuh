@@ -49,13 +49,45 @@ __device__ __forceinline__ void mma_16<__half>(float (&c)[4], const uint32_t (&a
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// two fp32 values as three 16-bit pairs: 24 bits and more, so nothing is left
 template <typename T>
-__device__ __forceinline__ void split_pair_16(float a, float b, uint32_t& hi, uint32_t& lo) { split_pair(a, b, hi, lo); }
+__device__ __forceinline__ void split3_pair_16(float a, float b, uint32_t (&t)[3]);
 template <>
-__device__ __forceinline__ void split_pair_16<__half>(float a, float b, uint32_t& hi, uint32_t& lo) {
-  const __half2 h = __floats2half2_rn(a, b);
-  const float2 f = __half22float2(h);
-  const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
+__device__ __forceinline__ void split3_pair_16<__nv_bfloat16>(float a, float b, uint32_t (&t)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    const float2 f = __bfloat1622float2(h);
+    a -= f.x;
+    b -= f.y;
+    t[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+template <>
+__device__ __forceinline__ void split3_pair_16<__half>(float a, float b, uint32_t (&t)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    a -= f.x;
+    b -= f.y;
+    t[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+// infinities as the largest finite values: the lower terms of a split are zero or of either sign
+template <typename T>
+__device__ __forceinline__ uint32_t finite_pair_16(uint32_t v);
+template <>
+__device__ __forceinline__ uint32_t finite_pair_16<__nv_bfloat16>(uint32_t v) {
+  const uint32_t top = 0x7f7f7f7fu, low = 0xff7fff7fu;
+  const __nv_bfloat162 x = __hmax2(__hmin2(*reinterpret_cast<const __nv_bfloat162*>(&v), *reinterpret_cast<const __nv_bfloat162*>(&top)),
+                                   *reinterpret_cast<const __nv_bfloat162*>(&low));
+  return *reinterpret_cast<const uint32_t*>(&x);
+}
+template <>
+__device__ __forceinline__ uint32_t finite_pair_16<__half>(uint32_t v) {
+  const uint32_t top = 0x7bff7bffu, low = 0xfbfffbffu;
+  const __half2 x = __hmax2(__hmin2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&top)),
+                            *reinterpret_cast<const __half2*>(&low));
+  return *reinterpret_cast<const uint32_t*>(&x);
 }
