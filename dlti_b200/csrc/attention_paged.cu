@@ -599,8 +599,8 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const PagedParams p, i
         }
       write(r, i - r * p.vdim, gm, gl, a);
     }
-    __syncwarp();                                  // nobody leaves while its shared memory is read; nothing has to be released
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    __syncwarp();
+    cluster_sync_all();                            // nobody leaves before the others have read its shared memory
   }
 }
 
