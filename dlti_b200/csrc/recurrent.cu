@@ -43,12 +43,16 @@ __device__ __forceinline__ float log_forget_gate(float z, float cap) { return -s
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
 
 // One token per sequence (decode rows). What bounds it is the state, read and written once; the token-by-token form below spends a
-// CTA of its own, with its three barriers and its loads of q and k, on every 32 columns, which left HBM at half its rate. Here a
-// lane owns V consecutive columns (one 16-byte access at V = 4), so the CTAs of an SM have 128 KB of the state in flight. 64 rows of
-// 8 heads of 128 x 256 (134 MB read and written): 43 -> 27 us, 5.0 TB/s. The order of all sums is that of the token-by-token form.
+// CTA of its own, with its three barriers and its loads of q and k, on every 32 columns. Here a lane owns V consecutive columns, so
+// the CTAs of an SM have 64 KB of the state in flight or more. States that come from HBM, us with the token-by-token form -> now: 8 heads of
+// 128 x 256 (mLSTM) 1 row 4.1 -> 3.6, 4 rows 5.6 -> 5.7, 16 rows 14.0 -> 9.0, 64 rows 47 -> 28; 64 heads of 128 x 64 1 row 3.5 -> 2.7, 4 rows 6.2 ->
+// 5.4, 16 rows 18.7 -> 15.0, 64 rows 75 -> 47 (268 MB read and written). The order of all sums is that of the token-by-token form. The
+// next kernel may start after the wait, not before it (griddep_pass): 256 CTAs take 5.7 instead of 6.3 us, as if the CTAs that already wait
+// on the SMs made these spread less evenly.
 template <typename T, int NR, int V, bool ML>
-__global__ void __launch_bounds__(256, NR * V <= 32 ? 4 : 2) scan_step_kernel(const ScanParams p, int blocks, int conv_parts) {
-  griddep_pass();
+__global__ void __launch_bounds__(256, step_ctas(NR, V)) scan_step_kernel(const ScanParams p, int blocks, int conv_parts) {
+  griddep_wait();
+  griddep_launch();
   const int s = p.seq0 + blockIdx.z;
   if ((int)blockIdx.x >= blocks) {
     if (blockIdx.y == 0) conv_tail<T>(p, s, blockIdx.x - blocks, conv_parts);
@@ -65,10 +69,7 @@ __global__ void __launch_bounds__(256, NR * V <= 32 ? 4 : 2) scan_step_kernel(co
 #pragma unroll
   for (int i = 0; i < NR; ++i) {
     const bool ok = live && colok && warp * NR + i < p.N;
-    if constexpr (V == 4) {
-      const float4 x = ok ? *reinterpret_cast<const float4*>(st + (long long)i * p.P) : make_float4(0.f, 0.f, 0.f, 0.f);
-      S[i][0] = x.x; S[i][1] = x.y; S[i][2] = x.z; S[i][3] = x.w;
-    } else if constexpr (V == 2) {
+    if constexpr (V == 2) {
       const float2 x = ok ? *reinterpret_cast<const float2*>(st + (long long)i * p.P) : make_float2(0.f, 0.f);
       S[i][0] = x.x; S[i][1] = x.y;
     } else {
@@ -83,6 +84,7 @@ __global__ void __launch_bounds__(256, NR * V <= 32 ? 4 : 2) scan_step_kernel(co
     if (p.silu) f = Cvt<T>::to_f(Cvt<T>::from_f(silu_f(f)));
     return f;
   };
+  constexpr int GATES = 224;                               // in a warp without loads of q and k (up to 128 rows), which would wait for the gates
   constexpr int NV = (NR + 31) / 32;                       // entries of n per lane
   const int slices = (p.P + 31) / 32;                      // every slice of 32 columns has its own n and m; they are equal
   float nv[NV], m = 0.f;
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(256, NR * V <= 32 ? 4 : 2) scan_step_kernel(co
       nv[i] = (live && lane + 32 * i < NR && r < p.N) ? vec[r] : 0.f;
     }
   }
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == GATES) {
     if constexpr (ML) {
       if (live) m = vec[p.N];
       const float zi = p.gates[row * p.g_ld + h] + p.gate_b[h], zf = p.gates[row * p.g_ld + p.heads + h] + p.gate_b[p.heads + h];
@@ -151,8 +153,7 @@ __global__ void __launch_bounds__(256, NR * V <= 32 ? 4 : 2) scan_step_kernel(co
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
       if (warp * NR + i >= p.N) break;
-      if constexpr (V == 4) *reinterpret_cast<float4*>(st + (long long)i * p.P) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
-      else if constexpr (V == 2) *reinterpret_cast<float2*>(st + (long long)i * p.P) = make_float2(S[i][0], S[i][1]);
+      if constexpr (V == 2) *reinterpret_cast<float2*>(st + (long long)i * p.P) = make_float2(S[i][0], S[i][1]);
       else st[(long long)i * p.P] = S[i][0];
     }
   }
@@ -166,7 +167,7 @@ __global__ void __launch_bounds__(256, NR * V <= 32 ? 4 : 2) scan_step_kernel(co
           const int r = warp * NR + lane + 32 * i;
           if (lane + 32 * i < NR && r < p.N) vec[x * (p.N + 1) + r] = nv[i];
         }
-        if (threadIdx.x == 0) vec[x * (p.N + 1) + p.N] = m;
+        if (threadIdx.x == GATES) vec[x * (p.N + 1) + p.N] = m;
       }
     }
   }
@@ -195,10 +196,8 @@ int launch_step(const ScanParams& p, int nseq, cudaStream_t st) {
 }
 template <typename T, int NR, bool ML>
 int dispatch_step(const ScanParams& p, int nseq, cudaStream_t st) {
-  constexpr int MOST = NR <= 16 ? 4 : (NR == 32 ? 2 : 1);
-  const int V = step_columns(p.P, MOST, (long long)p.heads * nseq, p.state);
-  if constexpr (MOST >= 4) if (V == 4) return launch_step<T, NR, 4, ML>(p, nseq, st);
-  if constexpr (MOST >= 2) if (V == 2) return launch_step<T, NR, 2, ML>(p, nseq, st);
+  const int V = step_columns(NR, p.P, (long long)p.heads * nseq, p.state);
+  if constexpr (NR <= 32) if (V == 2) return launch_step<T, NR, 2, ML>(p, nseq, st);
   return launch_step<T, NR, 1, ML>(p, nseq, st);
 }
 

@@ -42,10 +42,12 @@ __device__ __forceinline__ void conv_tail(const Params& p, int s, int part, int 
     }
 }
 
-// Columns per lane: as many as the states' alignment allows, as long as no lane stays idle and the SMs have a CTA each.
-inline int step_columns(int P, int most, long long heads, const void* state) {
-  for (int V = most; V > 1; V /= 2)
-    if (P % V == 0 && P > 16 * V && ((P + 32 * V - 1) / (32 * V)) * heads >= dlti_num_sms() && (reinterpret_cast<uintptr_t>(state) & (4 * V - 1)) == 0)
-      return V;
-  return 1;
+// Decode rows: columns per lane (V) of the kernels that move a state of 8 NR rows by N columns, and the CTAs that an SM holds of them
+// (registers). Two columns where the CTAs of one are more than one wave, and an even, aligned P allows it; four were never better. us
+// at V = 1 / 2 / 4: 16 heads of 128 x 128, 8 rows (512 CTAs at V = 1) 5.4 / 6.8 / 6.9, 16 rows (1024) 9.3 / 8.2 / 8.7, 64 rows 29.7 / 25.7 /
+// 28.0; mLSTM, 8 heads of 128 x 256, 64 rows 43.3 / 27.8 / 29.6; 256 rows of a state, 512 CTAs 10.1 / 8.8.
+__host__ __device__ constexpr int step_ctas(int NR, int V) { return NR * V <= 16 ? 4 : (NR * V == 32 ? (NR == 32 ? 3 : 4) : 2); }
+inline int step_columns(int NR, int P, long long heads, const void* state) {
+  const bool fits = NR <= 32 && P % 2 == 0 && P > 32 && (reinterpret_cast<uintptr_t>(state) & 7) == 0;
+  return fits && (P + 31) / 32 * heads > (long long)step_ctas(NR, 1) * dlti_num_sms() ? 2 : 1;
 }

@@ -24,8 +24,8 @@ def _act(x, device, dtype):
     return out.copy_(x)
 
 
-# four, two and one column per lane; last blocks and last rows partly filled; every row count of a warp
-SIZES = [(4, 128, 128, 40), (4, 128, 256, 40), (8, 30, 132, 40), (4, 72, 64, 40), (4, 20, 44, 80), (4, 128, 70, 40), (8, 256, 96, 40), (3, 64, 33, 60),
+# two columns and one per lane, on both sides of a wave of CTAs; last blocks and last rows partly filled; every row count of a warp
+SIZES = [(8, 128, 70, 40), (4, 20, 44, 160), (8, 60, 33, 80), (4, 200, 100, 27), (4, 200, 100, 28), (2, 128, 64, 148), (2, 128, 64, 149), (4, 128, 128, 40), (4, 128, 256, 40), (8, 30, 132, 40), (4, 72, 64, 40), (4, 20, 44, 80), (4, 128, 70, 40), (8, 256, 96, 40), (3, 64, 33, 60),
          (2, 300, 40, 80), (2, 128, 128, 3)]
 
 
