@@ -32,15 +32,19 @@ constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr int NUM_THREADS = 192;
 
-// Stages of the ring. Stream-K (decode): 120 KB in flight per SM cover HBM's latency, and what is left of the shared memory lets the
-// kernels around it start beside it; with 8 stages a step of 64 rows of 12 Llama layers of width 2048 took 856 us instead of 806
-// (6: 815; 4: 930).
-template <int BN, bool SK = false>
+// Stages of the ring. Decode steps of more than 4 rows (SHORT): 120 KB in flight per SM cover HBM's latency, and what is left of the
+// shared memory lets the kernels around it start beside it; a step of 64 rows of 12 Llama layers of width 2048 takes 806 us with 5 stages, 815
+// with 6, 856 with 8 and 930 with 4. With fewer rows those kernels are small and the weights are all there is: 5 / 8 stages, us a step, one row
+// of 4 Llama layers of width 4096 494 / 475, of a Logozen layer of 4096 352 / 338, of 8 Llama layers of 2048 418 / 412, of a Latanex layer of 2048
+// 177 / 171; 4 rows 435 / 435, of a Sigosun layer of 4096 398 / 384; 8 rows 471 / 457 (Llama, 4096) and 426 / 433 (2048), of Sigosun and Logozen
+// layers of 2048 192 / 195 and 280 / 284; 16 rows 457 / 453 (4096), 430 / 434 (2048).
+constexpr int DEEP_ROWS = 4;
+template <int BN, bool SHORT = false>
 struct Cfg {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128 ? (SK ? 4 : 6) : (SK ? 5 : 8));
+  static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128 ? (SHORT ? 4 : 6) : (SHORT ? 5 : 8));
   static constexpr int TMEM_COLS = 2 * BN;
   static constexpr int BAR_BYTES = 256;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + 1024;
@@ -151,14 +155,14 @@ struct SegIter {
   }
 };
 
-template <int BN, bool A_MN, bool B_MN, bool GATHER, bool PUSH, bool SK = false>
+template <int BN, bool A_MN, bool B_MN, bool GATHER, bool PUSH, bool SK = false, bool DEEP = false>
 __global__ void __launch_bounds__(NUM_THREADS + (GATHER ? GATHER_THREADS : 0), 1)
 gemm_tcgen05_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmA,
                     const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmA2,
                     const __grid_constant__ CUtensorMap tmB2,
                     const __grid_constant__ CUtensorMap tmBL, const GatherParams gp) {
-  using C_ = Cfg<BN, SK>;
+  using C_ = Cfg<BN, SK && !DEEP>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t bar_base = smem_base + C_::STAGES * C_::STAGE_BYTES;
@@ -530,27 +534,27 @@ inline int get_tmap(CUtensorMap* out, const void* base, uint64_t inner, uint64_t
   return dlti_get_tmap(out, base, inner, outer, ld, bi, bo);
 }
 
-template <int BN, bool A_MN, bool B_MN, bool GATHER, bool PUSH = false, bool SK = false>
+template <int BN, bool A_MN, bool B_MN, bool GATHER, bool PUSH = false, bool SK = false, bool DEEP = false>
 int launch(const GemmParams& p, const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& a2,
            const CUtensorMap& b2, const CUtensorMap& bl, const GatherParams& gp, int grid,
            cudaStream_t stream) {
-  using C_ = Cfg<BN, SK>;
+  using C_ = Cfg<BN, SK && !DEEP>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!configured[dev & 63]) {
-    DLTI_CUDA_CHECK(cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, A_MN, B_MN, GATHER, PUSH, SK>,
+    DLTI_CUDA_CHECK(cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, A_MN, B_MN, GATHER, PUSH, SK, DEEP>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          C_::SMEM_BYTES));
     configured[dev & 63] = true;
   }
   if constexpr (SK || PUSH) {
-    DLTI_CUDA_CHECK(dlti_launch_pdl(SK ? p.N : p.M, gemm_tcgen05_kernel<BN, A_MN, B_MN, GATHER, PUSH, SK>, dim3(grid),
+    DLTI_CUDA_CHECK(dlti_launch_pdl(SK ? p.N : p.M, gemm_tcgen05_kernel<BN, A_MN, B_MN, GATHER, PUSH, SK, DEEP>, dim3(grid),
                                     dim3(NUM_THREADS), C_::SMEM_BYTES, stream, p, a, b, a2, b2, bl, gp));
     dlti_count_launch();
     return 0;
   }
-  gemm_tcgen05_kernel<BN, A_MN, B_MN, GATHER, PUSH, SK>
+  gemm_tcgen05_kernel<BN, A_MN, B_MN, GATHER, PUSH, SK, DEEP>
       <<<grid, NUM_THREADS + (GATHER ? GATHER_THREADS : 0), C_::SMEM_BYTES, stream>>>(p, a, b, a2, b2, bl, gp);
   dlti_count_launch();
   return (int)cudaGetLastError();
@@ -684,6 +688,7 @@ static int gemm_impl(const void* A, const void* B, void* C, const void* R, int M
     if (items < grid) grid = (int)items;
     if (bn == 256) return launch<256, false, false, false, false, true>(p, ta, tb, ta2, tb2, tbl, gp, grid, stream);
     if (bn == 128) return launch<128, false, false, false, false, true>(p, ta, tb, ta2, tb2, tbl, gp, grid, stream);
+    if (p.N <= DEEP_ROWS) return launch<64, false, false, false, false, true, true>(p, ta, tb, ta2, tb2, tbl, gp, grid, stream);
     return launch<64, false, false, false, false, true>(p, ta, tb, ta2, tb2, tbl, gp, grid, stream);
   }
   if (push_world > 0) {
