@@ -744,10 +744,14 @@ DLTI_API int dlti_attn_paged_decode(const void* q, long long q_ld, int q_hd, con
   HEAD_DISPATCH(kd, vd, launch_decode, p, splits, ws, st);
 }
 
-// bf16 or fp16, heads of 128: decode attention of a model whose query heads share key / value heads (see dlti_paged_decode)
-int dlti_paged_decode_groups(const void* q, long long q_ld, const void* kc, const void* vc, const int* tables, int max_blocks, const int* ctx,
+// dlti_paged_decode for query heads that share key / value heads, which are read once for a group: bf16 or fp16, heads of 128
+DLTI_API int dlti_paged_decode_groups(const void* q, long long q_ld, const void* kc, const void* vc, const int* tables, int max_blocks, const int* ctx,
                              int batch, int bs, int H, int G, float scale, int splits, float* ws, void* out, long long o_ld, int dtype,
                              cudaStream_t st) {
+  if (batch <= 0) return 0;
+  if (G < 1 || H % G || splits < 1 || batch > 65535 || bs < 1 || q_ld % 2 || (reinterpret_cast<uintptr_t>(q) & 3) || (splits > 8 && !ws) ||
+      ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15))
+    return DLTI_ERR_BAD_ARG;
   PagedParams p{q, q_ld, 128, kc, vc, 128, 128, tables, max_blocks, bs, ctx, nullptr, nullptr, nullptr, 0, H, G, 128, 128, 0, 0, scale, 0.f,
                 nullptr, out, o_ld, batch, nullptr, nullptr, 0, nullptr, 0};
   if (dtype == DLTI_BF16) return launch_decode_t<bf16, 128, 128, true>(p, splits, ws, st);

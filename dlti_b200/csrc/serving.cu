@@ -10,11 +10,6 @@
 // (reference requirements.txt:18) and ships no serving code.
 #include "common.cuh"
 
-// attention_paged.cu
-int dlti_paged_decode_groups(const void* q, long long q_ld, const void* kc, const void* vc, const int* tables, int max_blocks, const int* ctx,
-                             int batch, int bs, int H, int G, float scale, int splits, float* ws, void* out, long long o_ld, int dtype,
-                             cudaStream_t st);
-
 namespace {
 
 constexpr int HD = 128;
@@ -489,11 +484,6 @@ DLTI_API int dlti_paged_decode(const void* q, long long q_stride, const void* k_
                                cudaStream_t st) {
   if (batch <= 0) return 0;
   if (hd != HD || H % KV || splits < 1) return DLTI_ERR_BAD_ARG;
-  // Query heads that share a key / value head read it once between them, on the tensor cores; paged_decode_kernel would read it for
-  // each of them. Llama layers of 16 heads on 4: a step of 64 x 120 keys, 12 layers, 811 -> 777 us, of 8 x 1000, 4 layers, 290 -> 284; with
-  // few requests the head-by-head kernel has the more CTAs: 1 x 4000 272 against 282.
-  if (H > KV && (long long)batch * H >= 64) return dlti_paged_decode_groups(q, q_stride, k_cache, v_cache, block_tables, max_blocks, ctx_lens, batch, block_size, H, KV, scale,
-                                              splits, workspace, out, out_stride, dtype, st);
   float* part_o = workspace;
   float* part_ml = workspace + (long long)batch * H * splits * HD;
   dim3 grid(splits, H, batch), g2(H, batch);

@@ -84,9 +84,19 @@ _ws_retired: list = []
 
 def decode_splits(ctas: int, reach: int) -> int:
     """CTAs over which the grouped decode attention cuts contexts of up to `reach` keys (tiles of 64) when one each would be `ctas`: one
-    wave of three per SM. Up to 8 are a cluster and merge by themselves; more are combined by a second kernel (8 CTAs with two tiles
-    each in their place took as long: 4 sequences of 1000 keys)."""
+    wave of three per SM. Up to 8 are a cluster and merge by themselves; more are combined by a second kernel."""
     return max(1, min(32, 3 * 148 // max(1, ctas), -(-reach // 64)))
+
+
+def heads_together(batch: int, H: int, KV: int, reach: int) -> bool:
+    """Whether one CTA serves the query heads of a group (dlti_paged_decode_groups) or each head is by itself (dlti_paged_decode), for contexts
+    of up to `reach` keys. Together they read keys and values once, on the tensor cores, but start later: a CTA needs 70 KB of shared memory.
+    us a step of 4 Llama layers of 16 heads, apart / together: contexts of 180 keys with a reach of 192, 4 heads a group, 4 rows 234 / 240, 16 rows
+    234 / 238, 64 rows 323 / 290 (2 a group 328 / 334, 16 a group 318 / 298); reach 256, 4 rows 242 / 235, 16 rows 241 / 233, 64 rows 342 / 299 (2 a
+    group 346 / 350, 16 a group 339 / 294); reach 512, 4 rows 254 / 240, 16 rows 264 / 251, 64 rows 416 / 335; 1000 keys, 4 rows 256 / 248, 16
+    rows 322 / 262; 4000 keys, 2 rows 272 / 287, 8 rows 425 / 299. Where contexts of 100 keys meet a reach of 1024, 4 rows lose (228 / 237) and
+    32 win (254 / 244): the lengths are not known when a step is captured."""
+    return H > KV and (batch * H >= 64 if reach >= 256 else batch * H >= 1024 and H >= 4 * KV)
 
 
 def paged_decode(q, k_cache, v_cache, block_tables, ctx_lens, H, KV, hd, scale=None, out=None,
@@ -106,10 +116,19 @@ def paged_decode(q, k_cache, v_cache, block_tables, ctx_lens, H, KV, hd, scale=N
         out = torch.empty((B, H * hd), dtype=q.dtype, device=q.device)
     bs = k_cache.shape[1]
     mc = max_ctx if max_ctx is not None else block_tables.shape[1] * bs
+    if hd == 128 and heads_together(B, H, KV, mc):
+        # never more than a cluster: with the second kernel 4 rows of 100 keys take 254 instead of 236 us a step where 4096 are allowed, 8 rows
+        # of 4000 keys 344 instead of 299 (4 heads a group), 283 instead of 288 (16)
+        splits = min(8, decode_splits(B * KV * -(-(H // KV) // 16), mc))
+        f = _lib.fn("dlti_paged_decode_groups", [_V, _L, _V, _V, _V, _I, _V, _I, _I, _I, _I, _F, _I, _V, _V, _L, _I, _V])
+        _lib.check(f(_lib.ptr(q), q.stride(0), _lib.ptr(k_cache), _lib.ptr(v_cache), _lib.ptr(block_tables),
+                     block_tables.shape[1], _lib.ptr(ctx_lens), B, bs, H, KV, float(scale), splits,
+                     None, _lib.ptr(out), out.stride(0), _lib.dtype_code(q.dtype), _lib.stream_ptr()),
+                   "paged_decode_groups")
+        return out
     # enough CTAs (128 threads each, ~4 resident per SM) to fill the machine: short contexts are latency-bound,
     # so small batches are cut into more KV splits
-    grouped = H > KV and B * H >= 64              # the kernel that dlti_paged_decode takes
-    splits = decode_splits(B * KV * -(-(H // KV) // 16), mc) if grouped else max(1, min(16, -(-(4 * 148) // max(1, B * H)), (mc + 255) // 256))
+    splits = max(1, min(16, -(-(4 * 148) // max(1, B * H)), (mc + 255) // 256))
     need = _lib.fn("dlti_paged_decode_workspace_floats", [_I, _I, _I], C.c_int)(B, H, splits)
     key = str(q.device)
     ws = _ws.get(key)

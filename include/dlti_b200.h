@@ -341,6 +341,11 @@ int dlti_paged_decode(const void* q, long long q_stride, const void* k_cache, co
                       const int* block_tables, int max_blocks, const int* ctx_lens, int batch,
                       int block_size, int H, int KV, int hd, float scale, int splits, float* workspace,
                       void* out, long long out_stride, int dtype, dlti_stream_t stream);
+/* the same for H query heads on G key / value heads of 128, which are read once for a group; workspace: see dlti_paged_decode (up to 8
+ * splits merge without it) */
+int dlti_paged_decode_groups(const void* q, long long q_ld, const void* kc, const void* vc, const int* tables, int max_blocks, const int* ctx,
+                             int batch, int bs, int H, int G, float scale, int splits, float* ws, void* out, long long o_ld, int dtype,
+                             dlti_stream_t stream);
 /* temperature / top-k / top-p / greedy sampling, one CTA per sequence, counter-based RNG keyed by
  * (seeds[b], step); out_logprob may be NULL */
 int dlti_sample(const void* logits, long long ld, int batch, int V, const float* temperature,

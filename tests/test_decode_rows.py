@@ -105,11 +105,12 @@ def test_prompts_in_segments(kind, N, P, lens, carried, monkeypatch):
 @pytest.mark.parametrize("dtype,tol", [(BF16, 4e-3), (torch.float16, 6e-4)])       # outputs rounded to 8 and 11 bits
 @pytest.mark.parametrize("max_ctx", [64, 400, 4096])                               # one CTA, a cluster, more than a cluster
 @pytest.mark.parametrize("H,KV,bs", [(4, 2, 16), (8, 2, 16), (16, 1, 24), (20, 1, 16), (51, 3, 16)])
-def test_decode_attention_of_shared_heads(H, KV, bs, max_ctx, dtype, tol):
+def test_decode_attention_of_shared_heads(H, KV, bs, max_ctx, dtype, tol, monkeypatch):
     from dlti_b200.ops import serving as S
+    monkeypatch.setattr(S, "heads_together", lambda *a: True)        # also at sizes that go head by head
     g = torch.Generator().manual_seed(H)
     ctx = [c for c in (1, 15, 63, 64, 65, 129, 400, 700, 4096) if c <= max_ctx]
-    ctx += [37] * (-(-64 // H) - len(ctx))                        # the rows from which the heads of a group go together
+    ctx += [37] * (-(-64 // H) - len(ctx))
     nb = [-(-c // bs) for c in ctx]
     tables, kc, vc = torch.zeros(len(ctx), max(nb), dtype=torch.int32), *(torch.randn(sum(nb), bs, KV, 128, generator=g).to(dtype) for _ in range(2))
     perm, at = torch.randperm(sum(nb), generator=g).int(), 0

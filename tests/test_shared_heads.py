@@ -27,6 +27,12 @@ def _paged(rows, bs=16):
     return kc.cuda(), vc.cuda(), tables.cuda(), torch.tensor([len(k) for k, _ in rows], dtype=torch.int32).cuda()
 
 
+@pytest.fixture(autouse=True)
+def together(monkeypatch):
+    """At every size, not where it pays alone."""
+    monkeypatch.setattr(S, "heads_together", lambda batch, H, KV, reach: H > KV)
+
+
 def _run(q, rows, H, max_ctx, alone=False):
     kc, vc, tables, ctx = _paged(rows)
     KV = kc.shape[2]
@@ -74,8 +80,8 @@ def test_no_further_from_64_bits_than_head_by_head(dtype, H, KV, longest):
     rows = [tuple(torch.randn(n, KV, 128, generator=g).to(dtype) for _ in range(2)) for n in [longest - longest * i // 12 for i in range(8)]]
     q = (2 * torch.randn(8, H * 128, generator=g)).to(dtype)
     want = _exact(q, rows, H)
-    together, alone = ((_run(q, rows, H, longest, alone) - want).norm() for alone in (False, True))
-    assert together <= 1.002 * alone                   # both are the rounding of the output, fp32 errors move a few ties
+    error, by_head = ((_run(q, rows, H, longest, alone) - want).norm() for alone in (False, True))
+    assert error <= 1.002 * by_head                   # both are the rounding of the output, fp32 errors move a few ties
 
 
 @pytest.mark.parametrize("dtype", [BF16, F16])
@@ -91,3 +97,24 @@ def test_infinite_values(dtype, max_ctx):
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
     ok = want.isfinite()
     assert (got - want)[ok].norm() <= (4e-3 if dtype == BF16 else 6e-4) * want[ok].norm()      # outputs rounded to 8 and 11 bits
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16])
+@pytest.mark.parametrize("H,KV,splits", [(8, 4, 1), (16, 4, 3), (32, 2, 16)])
+def test_the_entry_for_single_heads_stays_itself(dtype, H, KV, splits):
+    """dlti_paged_decode gives shared heads the arithmetic of heads with keys and values of their own, at any number of rows."""
+    g = torch.Generator().manual_seed(H)
+    rows = [tuple(torch.randn(n, KV, 128, generator=g).to(dtype) for _ in range(2)) for n in [700 - 40 * i for i in range(16)]]
+    q = torch.randn(16, H * 128, generator=g).to(dtype).cuda()
+    got = []
+    for share in (H // KV, 1):
+        kc, vc, tables, ctx = _paged(rows)
+        kc, vc = (x.repeat_interleave(H // KV // share, 2).contiguous() for x in (kc, vc))
+        out, ws = torch.empty_like(q), torch.empty(16 * H * splits * 130, device="cuda")
+        V, I, L = S._V, S._I, S._L
+        f = S._lib.fn("dlti_paged_decode", [V, L, V, V, V, I, V, I, I, I, I, I, S._F, I, V, V, L, I, V])
+        p = S._lib.ptr
+        S._lib.check(f(p(q), q.stride(0), p(kc), p(vc), p(tables), tables.shape[1], p(ctx), 16, 16, H, kc.shape[2], 128, 128 ** -0.5, splits, p(ws), p(out),
+                       out.stride(0), S._lib.dtype_code(dtype), S._lib.stream_ptr()), "paged_decode")
+        got.append(out.cpu())
+    assert torch.equal(*got)
