@@ -12,6 +12,7 @@ scheduler + block manager (SP:vllm/v1/core/sched/scheduler.py), async scheduling
 """
 from __future__ import annotations
 
+import math
 import time
 import uuid
 from array import array
@@ -116,12 +117,25 @@ def chunk_pieces(cu, starts, tables, bs: int, chunk: int, pack_prefix: int = 4, 
     return np.concatenate([np.asarray(x, dtype=np.int32) for x in arrays]), len(q0), longest, cue[-1], prefix
 
 
+def _int_array(toks) -> np.ndarray:
+    """int64 array of whole numbers: `array` reads a list of Python ints faster than numpy does."""
+    return np.frombuffer(array("q", toks if isinstance(toks, list) else list(toks)), dtype=np.int64) if len(toks) else np.empty(0, dtype=np.int64)
+
+
 def _id_array(toks) -> np.ndarray:
-    """int64 array of token ids: `array` reads a list of Python ints faster than numpy does."""
+    """int64 array of token ids, for a look at their range: what is outside (below zero by less than one, too) stays outside."""
     try:
-        return np.frombuffer(array("q", toks if isinstance(toks, list) else list(toks)), dtype=np.int64) if len(toks) else np.empty(0, dtype=np.int64)
-    except (TypeError, OverflowError):                # not plain ints, or not 64 bits: what is outside stays outside
-        return np.asarray([min(max(int(t), -1), 1 << 62) for t in toks], dtype=np.int64)
+        return _int_array(toks)
+    except (TypeError, OverflowError):                # not plain ints, or not 64 bits
+        return np.asarray([math.floor(min(max(t, -1), 1 << 62)) for t in toks], dtype=np.int64)
+
+
+def _stored_ids(toks: list) -> np.ndarray:
+    """int64 array of the ids that a request holds."""
+    try:
+        return _int_array(toks)
+    except TypeError:
+        return np.asarray(toks, dtype=np.int64)
 
 
 class PackedStep:
@@ -367,7 +381,7 @@ class LLMEngine:
             for r in reqs[nd:]:
                 a, n = r.num_computed, r.chunk              # this step prefills tokens [a, a + n) of the sequence
                 own = given.get(id(r)) if given else None
-                ia.append(_id_array((r.prompt_ids + r.output_ids)[a:a + n]) if own is None else own)
+                ia.append(_stored_ids((r.prompt_ids + r.output_ids)[a:a + n]) if own is None else own)
                 ps.append(ar[a:a + n])
                 blk = np.asarray(r.blocks[:-(-(a + n) // bs)], dtype=np.int64)
                 allslots = (blk[:, None] * bs + ar[None, :bs]).reshape(-1)
@@ -680,13 +694,17 @@ class LLMEngine:
         order = decode + rest
         given = {}
         for r, toks, _ in order:
-            own = given[id(r)] = _id_array(toks)
+            own = _id_array(toks)
             if own.size and not (own.min() >= 0 and own.max() < self.cfg.vocab_size):
                 raise ValueError(f"request {r.request_id}: token outside the vocabulary of {self.cfg.vocab_size}")
             if r.num_computed + len(toks) > self.max_model_len:
                 raise ValueError(f"request {r.request_id}: longer than {self.max_model_len} tokens")
             if not self.sched._acquire(r, r.num_computed + len(toks)):
                 raise RuntimeError(f"request {r.request_id}: out of cache pages or state slots")
+            if len(r.prompt_ids) == r.num_computed and not r.output_ids:
+                given[id(r)] = own
+            else:                                    # a request with tokens that no step has run: its oldest ones come first
+                given.pop(id(r), None)
             r.prompt_ids.extend(toks)
             r.chunk = len(toks)
             r.status = "running"
