@@ -32,10 +32,18 @@ from .kv_cache import KVCache, KVSpec
 _FUSE_ACC = os.environ.get("DLTI_DECODE_FUSE_ACC", "1") == "1"    # A/B switch: consume the fp32 accumulators directly
 
 
+# gate_up product of prompts with SwiGLU in its epilogue: "1" always, "0" never, unset where it was measured (one GPU's rows)
+_PREFILL_FUSE_SWIGLU = os.environ.get("DLTI_SERVE_FUSE_SWIGLU", "")
 _TP_LARGE = os.environ.get("DLTI_TP_LARGE_RSAG", "1") == "1"          # prefill-sized steps: reduce-scatter + all-gather
 # how prefill-sized steps do it: "fused" = reduce-scatter in the row-parallel GEMM's epilogue (K10) and all-gather in
 # the next column-parallel GEMM's producer (K11); "pull" = the round-1 stand-alone pull-reduce-push kernel
 _TP_LARGE_MODE = os.environ.get("DLTI_TP_LARGE_MODE", "fused")
+
+
+def swiglu_in_epilogue(x) -> bool:
+    """Whether the gate_up product of the prompt rows x applies SwiGLU itself: 4 layers of 7B over 7400 prompt rows spent 517 us in the kernel
+    of its own, now 58 more in the GEMMs. Rows that live on several ranks (ShardedAct) keep the two kernels: not measured there."""
+    return _PREFILL_FUSE_SWIGLU == "1" or (_PREFILL_FUSE_SWIGLU != "0" and not isinstance(x, ShardedAct))
 
 
 class ShardedAct:
@@ -448,9 +456,7 @@ class ModelRunner:
                 xn = row_reduce(attn, lw["w_o"], lw["ln2"])
             if acc_path:
                 h = E.acc_swiglu(gemm_skinny_acc(xn, lw["w_gu"]), xn.dtype)
-            elif not skinny:
-                # SwiGLU in the CTA-pair GEMM's epilogue (falls back by itself): 4 layers of 7B over 7400 prompt rows spent 517 us
-                # in the kernel of its own, now 58 more in the GEMMs
+            elif not skinny and swiglu_in_epilogue(xn):     # falls back by itself
                 h = (gemm_swiglu(xn.rows(), lw["w_gu"], gather=xn.handle) if isinstance(xn, ShardedAct)
                      else gemm_swiglu(xn, lw["w_gu"]))
             else:
