@@ -749,7 +749,7 @@ static int tp_reduce_impl(const void* recv, long long slot_stride, int world, vo
 #define TRN(T, V)                                                                                                    \
   do {                                                                                                               \
     if (tb)                                                                                                          \
-      DLTI_CUDA_CHECK(dlti_launch_pdl(rows, tp_reduce_add_norm_kernel<T, V, true>, dim3((unsigned)rows), dim3(128), 0, \
+      DLTI_CUDA_CHECK(dlti_launch_pdl(dlti_peer_rows(rows), tp_reduce_add_norm_kernel<T, V, true>, dim3((unsigned)rows), dim3(128), 0, \
                                       st, (const T*)recv, slot_stride, world, (T*)residual, (const T*)w, (T*)y, d,   \
                                       eps, *tb));                                                                    \
     else                                                                                                             \

@@ -42,8 +42,8 @@ int dlti_num_sms();
 // path are launched with cudaLaunchAttributeProgrammaticStreamSerialization, so a kernel's prologue overlaps the
 // tail of its predecessor; every such kernel orders its global accesses behind griddep_wait(). Level 2 (set by
 // the serving engine, whose weights never change): the decode GEMM also requests its first weight tiles BEFORE
-// the wait — only valid when no earlier kernel still in flight writes the weight matrix. Level 0: plain stream
-// ordering. DLTI_PDL=0|1|2 in the environment or dlti_set_pdl(level).
+// the wait — only valid when none of the kernels in flight, which may be several before it (griddep_pass), writes the weight
+// matrix. Level 0: plain stream ordering. DLTI_PDL=0|1|2 in the environment or dlti_set_pdl(level).
 int dlti_pdl_enabled();
 
 // ---------------------------------------------------------------------------
@@ -70,6 +70,9 @@ int dlti_get_tmap_mn3d(CUtensorMap* out, const void* base, uint64_t N, uint64_t 
 // and 655 instead of 727 us on 6 Logozen layers; at 64 rows of 4 Llama-2-7B layers, where the weights take most of it, 678 and
 // 680 us. Larger steps fall back to plain stream ordering: their kernels fill the GPU.
 constexpr long long DLTI_PDL_MAX_ROWS = 256;
+// Kernels that exchange rows with other ranks were measured up to 32 rows that way; with more they follow the stream's order.
+constexpr long long DLTI_PDL_MAX_PEER_ROWS = 32;
+inline long long dlti_peer_rows(long long rows) { return rows <= DLTI_PDL_MAX_PEER_ROWS ? rows : DLTI_PDL_MAX_ROWS + 1; }
 // cluster > 1: CTAs of a cluster along x.
 template <typename... KArgs, typename... Args>
 inline cudaError_t dlti_launch_pdl_cluster(long long rows, int cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,

@@ -549,7 +549,7 @@ int launch(const GemmParams& p, const CUtensorMap& a, const CUtensorMap& b, cons
     configured[dev & 63] = true;
   }
   if constexpr (SK || PUSH) {
-    DLTI_CUDA_CHECK(dlti_launch_pdl(SK ? p.N : p.M, gemm_tcgen05_kernel<BN, A_MN, B_MN, GATHER, PUSH, SK, DEEP>, dim3(grid),
+    DLTI_CUDA_CHECK(dlti_launch_pdl(SK ? p.N : dlti_peer_rows(p.M), gemm_tcgen05_kernel<BN, A_MN, B_MN, GATHER, PUSH, SK, DEEP>, dim3(grid),
                                     dim3(NUM_THREADS), C_::SMEM_BYTES, stream, p, a, b, a2, b2, bl, gp));
     dlti_count_launch();
     return 0;
