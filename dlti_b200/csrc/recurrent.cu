@@ -414,8 +414,9 @@ __global__ void __launch_bounds__(chunk_threads(MODE), NT <= 128 ? 2 : 1) scan_c
   using L = ChunkSmem<NT, MODE>;
   using bf16 = __nv_bfloat16;
   const int sq = MODE == SEG_FULL ? blockIdx.z / p.segs : blockIdx.z, seg = MODE == SEG_FULL ? blockIdx.z - sq * p.segs : 0, s = p.seq0 + sq;
-  if ((int)blockIdx.x >= slices) {
-    if (blockIdx.y == 0 && seg == 0) conv_tail<bf16>(p, s, blockIdx.x - slices, conv_parts);
+  const int cells = slices * p.heads, h = (int)blockIdx.x / slices, slice = (int)blockIdx.x - h * slices;
+  if ((int)blockIdx.x >= cells) {                                // behind all others: see launch_chunk_mode
+    if (seg == 0) conv_tail<bf16>(p, s, blockIdx.x - cells, conv_parts);
     return;
   }
   extern __shared__ __align__(128) uint8_t smem[];
@@ -423,14 +424,14 @@ __global__ void __launch_bounds__(chunk_threads(MODE), NT <= 128 ? 2 : 1) scan_c
   long long row0;
   int n, start;
   seq_rows(p, s, row0, n, start);
-  const int h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c0 = blockIdx.x * CP, ncol = min(CP, p.P - c0), grp = h / p.rep;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c0 = slice * CP, ncol = min(CP, p.P - c0), grp = h / p.rep;
   const int slot = p.sslot[s];
   const int last_seg = MODE == WHOLE ? 0 : min((n - 1) / p.seg_len, p.segs - 1);       // the tokens [tb, te) are this CTA's
   if (MODE != WHOLE && (n <= 0 || seg > last_seg || (MODE == SEG_STATE && last_seg == 0))) return;
   const int tb = MODE == SEG_FULL ? seg * p.seg_len : 0;
   const int te = MODE == SEG_STATE ? last_seg * p.seg_len : (seg == last_seg ? n : tb + p.seg_len);
-  auto entry = [&](int i) { return p.seg_ws + ((((long long)sq * p.segs + i) * p.heads + h) * slices + blockIdx.x) * SegEntry<NT>::FLOATS; };
+  auto entry = [&](int i) { return p.seg_ws + ((((long long)sq * p.segs + i) * p.heads + h) * slices + slice) * SegEntry<NT>::FLOATS; };
   const bf16* q = reinterpret_cast<const bf16*>(p.q) + row0 * p.q_ld + (long long)grp * p.N;
   const bf16* k = reinterpret_cast<const bf16*>(p.k) + row0 * p.k_ld + (long long)grp * p.N;
   const bf16* v = reinterpret_cast<const bf16*>(p.v) + row0 * p.v_ld + (long long)h * p.P + c0;
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(chunk_threads(MODE), NT <= 128 ? 2 : 1) scan_c
   const float la_c = !ML && p.decay ? fmaxf(logf(p.decay[h]), -80.f) * LOG2E : 0.f;
   const float bias = ML ? p.gate_b[h] : (p.decay ? 0.f : p.dt_bias[h]);
   const float bias_f = ML ? p.gate_b[p.heads + h] : 0.f;
-  float* vecs = ML ? p.vec + (((long long)(slot < 0 ? 0 : slot) * p.heads + h) * slices + blockIdx.x) * (p.N + 1) : nullptr;
+  float* vecs = ML ? p.vec + (((long long)(slot < 0 ? 0 : slot) * p.heads + h) * slices + slice) * (p.N + 1) : nullptr;
   float m = 0.f;                                                 // warp PREP, mLSTM: log2 of the running maximum
   // warp PREP: step sizes and decays of the chunk at t0, two consecutive tokens a lane
   auto raw_dt = [&](int t0, float (&d)[4]) {                     // mLSTM: input gates, then forget gates
@@ -887,16 +888,17 @@ __global__ void __launch_bounds__(chunk_threads(MODE), NT <= 128 ? 2 : 1) scan_c
 
 // Segments per sequence: as many as fill the SMs with the CTAs that fit one of them side by side (two up to 128 rows of a state, one
 // above: shared memory), of at least 8 chunks. Two CTAs of an SM slow each other down, so that more than one per SM has to come with
-// three segments or more. 8192 tokens in 1 / 2 / 3 / 4 / 8 segments, us, heads of 128 x 128: 32 CTAs 339 / 243 / 208 / 189 / 185, 64 CTAs 341 /
-// 247 / 263 / 230 / 253, 96 CTAs 344 / 329 / 267 / 359 / 321, 128 CTAs 343 / 327 / 431 / 364 / 386 and, where a step size is computed, 354 / 353
-// / 460; 1024 tokens of 128 CTAs: 52 whole, 60 in two. Heads of 256 x 256, 4096 tokens: 64 CTAs 266 / 192 / 251, 96 CTAs 267 / 325 / 261.
+// three segments or more, or with a long sequence. 8192 tokens in 1 / 2 / 3 / 4 / 8 segments, us, heads of 128 x 128: 32 CTAs 339 / 243 / 208 /
+// 189 / 185, 64 CTAs 341 / 247 / 263 / 230 / 253, 96 CTAs 344 / 329 / 267 / 359 / 321, 128 CTAs 343 / 327 / 431 / 364 / 386, with q and k shared by
+// all heads 383 / 368; 128 CTAs with 4096 tokens 169 / 171, with 1024 52 / 60. Heads of 256 x 256, 4096 tokens: 64 CTAs 266 / 192 / 251, 96
+// CTAs 267 / 325 / 261.
 inline int scan_segments(int longest, int nseq, int heads, int N, int P) {
   const long long ctas = (long long)((P + CP - 1) / CP) * heads * nseq, sms = dlti_num_sms();
   const long long room = (N <= 128 ? 2 : 1) * sms / (ctas > 0 ? ctas : 1);
   const int most = longest / (8 * CQ);
   int segs = (int)(room < most ? room : most);
   segs = segs < 16 ? segs : 16;
-  return segs > 2 || (segs == 2 && 2 * ctas <= sms) ? segs : 1;
+  return segs > 2 || (segs == 2 && (2 * ctas <= sms || (room == 2 && longest >= 80 * CQ))) ? segs : 1;
 }
 
 template <int NT, bool ML, int MODE>
@@ -910,7 +912,9 @@ int launch_chunk_mode(const ScanParams& p, int nseq, int conv_parts, cudaStream_
     done[dev & 63] = true;
   }
   const int slices = (p.P + CP - 1) / CP;
-  scan_chunk_kernel<NT, ML, MODE><<<dim3(slices + conv_parts, p.heads, nseq * (MODE == SEG_FULL ? p.segs : 1)), chunk_threads(MODE), bytes, st>>>(p, slices, conv_parts);
+  // The few CTAs of the convolution's state come last: as a share of every head they would be CTAs that leave at once, and of the others some SMs
+  // get two and some none (8192 tokens, 64 heads of 128 x 64 that share q and k: 508 us instead of 383)
+  scan_chunk_kernel<NT, ML, MODE><<<dim3(slices * p.heads + conv_parts, 1, nseq * (MODE == SEG_FULL ? p.segs : 1)), chunk_threads(MODE), bytes, st>>>(p, slices, conv_parts);
   dlti_count_launch();
   return (int)cudaGetLastError();
 }

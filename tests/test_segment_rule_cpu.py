@@ -15,8 +15,8 @@ def _segments(longest, nseq, heads, N, P):
     return max(1, floats // per)
 
 
-# (longest, sequences, heads, N, P) -> segments on 148 SMs: by the room of the SMs, by the length, whole where two fit no SM of their own
-RULE = [((8192, 1, 16, 128, 128), 4), ((8192, 1, 24, 128, 128), 3), ((8192, 1, 32, 128, 128), 1), ((8192, 1, 64, 128, 64), 1), ((1024, 1, 16, 128, 128), 2),
+# (longest, sequences, heads, N, P) -> segments on 148 SMs: by the room of the SMs, by the length, whole where two fit no SM of their own and are short
+RULE = [((8192, 1, 16, 128, 128), 4), ((8192, 1, 24, 128, 128), 3), ((5119, 1, 32, 128, 128), 1), ((5120, 1, 64, 128, 64), 2), ((1024, 1, 16, 128, 128), 2),
         ((1024, 1, 24, 128, 128), 1), ((1023, 1, 4, 64, 64), 1), ((1 << 20, 1, 1, 64, 32), 16), ((8192, 2, 8, 256, 256), 1), ((8192, 1, 8, 256, 256), 2),
         ((8192, 1, 12, 256, 256), 1), ((8192, 1, 4, 200, 256), 4), ((8192, 1, 4, 300, 64), 1)]
 
