@@ -28,7 +28,7 @@ cmd = [sys.executable, "-m", "vllm.entrypoints.openai.api_server", "--model", d,
 if a.compile_mode is not None:
     cmd += ["--compilation-config", json.dumps({"mode": a.compile_mode})]
 env = dict(os.environ, VLLM_NO_USAGE_STATS="1", HF_HUB_OFFLINE="1", TRANSFORMERS_OFFLINE="1")
-log = open("gpurun_out/vllm_server.log", "w") if os.path.isdir("gpurun_out") else subprocess.DEVNULL
+log = open("results/vllm_server.log", "w") if os.path.isdir("results") else subprocess.DEVNULL
 srv = subprocess.Popen(cmd, env=env, stdout=log, stderr=subprocess.STDOUT, start_new_session=True)
 url = f"http://127.0.0.1:{a.port}"
 ok = False
@@ -52,8 +52,8 @@ try:
         res = asyncio.run(sweep(url, "llama2-7b", levels, input_len=512, output_len=128, vocab=cfg.vocab_size, extra=extra))
         out = {"impl": "standin-vllm", "tp": a.tp, "startup_s": startup_s, "compile_mode": a.compile_mode, "levels": res}
         print(json.dumps(out))
-        if os.path.isdir("gpurun_out"):
-            json.dump(out, open(f"gpurun_out/vllm_standin_tp{a.tp}.json", "w"), indent=1)
+        if os.path.isdir("results"):
+            json.dump(out, open(f"results/vllm_standin_tp{a.tp}.json", "w"), indent=1)
 finally:
     import signal
     try:

@@ -43,5 +43,5 @@ for B in [int(x) for x in a.batches.split(",")]:
                  "floor_ms": floor, "frac_of_hbm_floor": floor / ms})
     if info.rank == 0: print(json.dumps(rows[-1]), flush=True)
 if info.rank == 0:
-    os.makedirs("gpurun_out", exist_ok=True); json.dump(rows, open(f"gpurun_out/decode_bench_tp{info.world_size}.json", "w"), indent=1)
+    os.makedirs("results", exist_ok=True); json.dump(rows, open(f"results/decode_bench_tp{info.world_size}.json", "w"), indent=1)
 

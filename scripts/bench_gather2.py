@@ -67,5 +67,5 @@ for name, R, Cc in [("w_qkv", 12288, 4096), ("w_o", 4096, 4096), ("w_gu", 22016,
     if rank == 0: print(json.dumps({k: (round(v, 1) if isinstance(v, float) else v) for k, v in res.items()}), flush=True)
 fc.check_error()
 if rank == 0:
-    os.makedirs("gpurun_out", exist_ok=True); json.dump(rows_out, open(f"gpurun_out/gather2_w{world}.json", "w"), indent=1)
+    os.makedirs("results", exist_ok=True); json.dump(rows_out, open(f"results/gather2_w{world}.json", "w"), indent=1)
 comm.shutdown()

@@ -73,8 +73,8 @@ def main():
         print(json.dumps(res), flush=True)
         del a, w, out, dy, dx
         torch.cuda.empty_cache()
-    os.makedirs("gpurun_out", exist_ok=True)
-    json.dump(rows, open("gpurun_out/bench_gemm.json", "w"), indent=1)
+    os.makedirs("results", exist_ok=True)
+    json.dump(rows, open("results/bench_gemm.json", "w"), indent=1)
 
 
 if __name__ == "__main__":

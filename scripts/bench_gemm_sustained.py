@@ -2,7 +2,7 @@
 """Sustained (power-capped) GEMM throughput: each variant runs back to back for ~SECS seconds, which is how the
 kernels run inside a training step on a 1 kW B200 (the burst numbers of bench_gemm.py are taken before the
 power governor reacts). dlti CTA-pair kernel vs torch.matmul (cuBLAS) at the Llama-2-7B shapes, NT and NN,
-each measured twice in alternation. Writes gpurun_out/bench_gemm_sustained.json (or $OUT).
+each measured twice in alternation. Writes results/bench_gemm_sustained.json (or $OUT).
   SECS=1.5  STREAMK=-1|0|1 (stream_k argument of the pair kernel)  SHAPES=qkv,o,...  M=4096"""
 import json
 import os
@@ -70,8 +70,8 @@ def main():
         print(json.dumps(res), flush=True)
         del a, w, out, dy, dx
         torch.cuda.empty_cache()
-    os.makedirs("gpurun_out", exist_ok=True)
-    json.dump(rows, open(os.environ.get("OUT", "gpurun_out/bench_gemm_sustained.json"), "w"), indent=1)
+    os.makedirs("results", exist_ok=True)
+    json.dump(rows, open(os.environ.get("OUT", "results/bench_gemm_sustained.json"), "w"), indent=1)
 
 
 if __name__ == "__main__":

@@ -24,7 +24,7 @@ def main():
     ap.add_argument("--input_len", type=int, default=512)
     ap.add_argument("--output_len", type=int, default=128)
     ap.add_argument("--requests_per_level", type=int, default=None)
-    ap.add_argument("--out", type=str, default="gpurun_out/serving_bench.json")
+    ap.add_argument("--out", type=str, default="results/serving_bench.json")
     a = ap.parse_args()
     info, cfg, eng = build_engine(a)
     if info.rank != 0:

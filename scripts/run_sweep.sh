@@ -12,5 +12,5 @@ for S in $STAGES; do
   FLAG=--deepspeed_config; [ "$S" = "3" ] && FLAG=--deepspeed
   run training/train_deepspeed_zero$S.py $FLAG configs/ds_config_zero$S.json $COMMON --no_offload --output_dir /tmp/ckpt/z$S 2>&1 | grep -E "^\{'loss|Throughput|Tokens/sec|Error|error|Traceback" | tail -4
 done
-mkdir -p gpurun_out; cp results/training_metrics.csv gpurun_out/training_metrics_${N}gpu.csv
+cp results/training_metrics.csv results/training_metrics_${N}gpu.csv
 python scripts/compare_training.py 2>&1 | tail -30

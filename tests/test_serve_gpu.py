@@ -114,9 +114,8 @@ sys.exit(0 if same >= 0.9 * 12 * len(prompts) else 1)
 
 def test_chunked_prefill_gpu(tmp_path):
     """Opt-in chunked prefill (prefill_chunk > 0) on the GPU kernels: later chunks attend to the cached prefix through
-    the extended [prefix | chunk] layout. Runs in its own process: the path had only been exercised on the CPU
-    oracles when this test was written, and a device fault must not take the remaining tests with it. It has
-    passed on B200 since round 1, so a failure (or a timeout) fails the test."""
+    the extended [prefix | chunk] layout. Runs in its own process, so that an error of the device stays
+    there; a failure or a timeout fails the test."""
     import os
     import subprocess
     import sys
