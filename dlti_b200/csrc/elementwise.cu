@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(128) rmsnorm_bwd_kernel(const T* __restrict__ 
   const float rstd = rstd_in[row];
   const int4* rr = dres ? reinterpret_cast<const int4*>(dres + row * d) : nullptr;
   float g[VPT][8], xh[VPT][8];
-  // requested with the rest: behind the sum it would be a second trip to memory (4096 x 4096: 36.0 -> 33.8 us, 5.0 TB/s)
+  // requested with the rest: behind the sum it would be a second trip to memory (4096 x 4096: 36.0 -> 33.8 us for 134 MB, 4.0 TB/s)
   int4 rv[VPT];
   float dot = 0.f;
 #pragma unroll
