@@ -123,8 +123,12 @@ __device__ __forceinline__ void griddep_pass() {
   griddep_launch();
   griddep_wait();
 }
-// With few rows of a wide model the weights are all there is and the competition costs more than the launch: a step of one row of 6
-// Llama-2-7B layers takes 622 us in the other order and 628 in this one, 64 rows of 12 layers of width 2048 824 and 806 us.
+// Llama's kernels. With few rows of a wide model the weights are all there is and the competition costs more than the launch. us a step,
+// release first / wait first:
+// 4 layers of width 4096 1 row 479 / 473, 4 rows 442 / 435, 12 rows 453 / 450, 17 rows 480 / 480, 64 rows 615 / 620; of 8
+// layers of width 2048, where the launches weigh more: 1 row 400 / 416, 4 rows 423 / 432, 8 rows 431 / 433, 16 rows 446 / 439, 32 rows 455 /
+// 450, 64 rows 579 / 588. The other families' kernels release first at every size (one row of width 2048: Sigosun 175 / 184, Logozen 271 /
+// 273), but for those that say otherwise.
 __device__ __forceinline__ void griddep_pass(long long rows) {
   if (rows > 16) griddep_launch();
   griddep_wait();

@@ -118,3 +118,36 @@ def test_the_entry_for_single_heads_stays_itself(dtype, H, KV, splits):
                        out.stride(0), S._lib.dtype_code(dtype), S._lib.stream_ptr()), "paged_decode")
         got.append(out.cpu())
     assert torch.equal(*got)
+
+
+def test_a_whole_model_either_way(monkeypatch):
+    """A bf16 model answering through the engine, its heads together and apart, beside the whole sequences run as prompts: what two ways of
+    rounding 16-bit activations differ by."""
+    from dlti_b200.models.config import PRESETS
+    from dlti_b200.models.llama import ResidentWeights
+    from dlti_b200.serve.engine import LLMEngine
+    from dlti_b200.serve.model_runner import TPContext, TPWeights
+    from dlti_b200.serve.params import Request, SamplingParams
+    from dlti_b200.serve.tokenizer import ByteTokenizer
+    cfg, rows, calls = PRESETS["tiny-gqa"], 40, []
+    full = ResidentWeights.random_init(cfg, "cuda", BF16, seed=3)
+    for t in full.all_matrices():
+        t.mul_(4.0)
+    w = TPWeights(cfg, 0, 1, "cuda", BF16).load_from_full(full)
+    g = torch.Generator().manual_seed(2)
+    toks = [torch.randint(3, cfg.vocab_size, (20 + 9 * i,), generator=g).tolist() for i in range(rows)]
+    request = lambda i: Request(str(i), [], SamplingParams(temperature=0.0))
+    got = []
+    for way in (True, False, None):
+        monkeypatch.setattr(S, "heads_together", lambda *a: calls.append(way) or way)
+        eng = LLMEngine(cfg, w, TPContext(), ByteTokenizer(cfg.vocab_size), num_blocks=1200, max_model_len=512, max_num_seqs=rows, max_num_batched_tokens=8192)
+        if way is None:
+            got.append(eng.replay_step([(request(i), t, list(range(len(t) - 6, len(t)))) for i, t in enumerate(toks)]).view(rows, 6, -1))
+            break
+        reqs = [request(i) for i in range(rows)]
+        eng.replay_step([(r, t[:-6], []) for r, t in zip(reqs, toks)])
+        got.append(torch.stack([eng.replay_step([(r, [t[k - 6]], [0]) for r, t in zip(reqs, toks)]) for k in range(6)], 1))
+    assert {True, False} <= set(calls) and cfg.num_key_value_heads < cfg.num_attention_heads
+    error = lambda a, b: (a - b).double().norm() / b.double().norm()
+    apart = error(got[1], got[2])
+    assert apart < 0.05 and error(got[0], got[2]) < 1.3 * apart + 2 ** -9 and error(got[0], got[1]) < 0.05
